@@ -10,30 +10,36 @@
 //   level 0  the state at step t, streamed by TMA: u and d of a plane around
 //            the 60 x 13 output tile (one 68 x 17 x 1 x 6 box per plane;
 //            4-stage ring: planes q and q+1 held, two in flight) and the
-//            material coefficients of the 64 x 15 level-1 region (2 stages);
+//            material coefficients of the 64 x 15 level-1 region, which arrive
+//            on the barrier of the next plane;
 //   level 1  step t+1 on the 64 x 15 region (the tile, one cell of halo, one
 //            more column each side in z so z pairs stay aligned), written to
-//            a 3-slot shared-memory ring of planes;
-//   level 2  step t+2 on the output tile, read from the level-1 ring and
-//            written to global memory.
+//            a 4-slot shared-memory ring of planes;
+//   level 2  step t+2 on the output tile, written to global memory.
 //
 // The CTA marches along x: when level-0 plane q+1 lands, level 1 computes
 // plane q and level 2 plane q-1.  Fifteen consumer warps each own one
-// level-1 row of 32 z pairs (8-byte shared loads and stores for both cells,
-// packed .f32x2 arithmetic) and the same pairs at level 2, so the
-// coefficients carry over in registers; the x neighbours at x-1 of both
-// levels come from registers too (the centre values of the plane computed
-// before), which frees a level-0 stage as soon as level 1 has used it.  The
-// level-1 ring has a full and an empty mbarrier per slot (one arrival per
-// warp): level 2 of plane q-1 waits until every warp has written plane q-1
-// (it reads the rows above and below), and level 1 reuses a slot once every
-// warp has read it, so warps drift up to a plane apart instead of meeting at
-// a barrier; every wait is bounded and an abort stops each warp on its own.
-// Level-1 cells outside the grid interior are the zero shell.  Both levels
-// use lap7_pair, so two steps here equal two one-step launches bit for bit.
-// A pass reads buffer t mod 3 and writes buffer (t+2) mod 3.  Batched
-// launches give each solve its own tile shape; the force terms of push
-// tiles come from a shared-memory term buffer the producer fills.
+// level-1 row of 32 z pairs (packed .f32x2 arithmetic) and the same pairs at
+// level 2.  A thread walks its own column in registers at both levels (level
+// 0 of planes q-1 and q, level 1 of planes q-2, q-1 and q, the coefficients
+// of q-1) and takes the z neighbours from the lanes either side, so shared
+// memory serves only the rows either side, the column's next level-0 plane
+// and the coefficients: 30 eight-byte loads per pair and plane instead of
+// the 76 of reading every stencil point (shared-memory wavefronts 15.4 M
+// instead of 26 M in a launch at 192^3).
+//
+// Two waits per plane and warp.  The level-1 ring has one mbarrier per slot
+// (one arrival per warp, when its row of the plane is written); level 2 of
+// plane q-1 waits for that plane.  Four slots need no barrier for their
+// reuse: a warp that has seen plane q-2 complete knows that every warp has
+// left iteration q-3, the last to read the slot plane q goes to.  With a
+// barrier of its own for the coefficients and one for the reuse of a slot
+// (four waits per plane) a quarter of the kernel's instructions were waits.
+// Columns in registers and two waits: 104 instead of 115 us per launch at
+// 192^3, 1.12x on a batch of 24 solves of 64..160 x 64..160 x 64..224 cells.
+// Every wait is bounded and an abort stops each warp on its own.  Force
+// terms of push tiles come from a shared-memory term buffer the producer
+// fills.
 //
 // It moves about 30 bytes of DRAM traffic per cell-step (u, d in and out
 // once per two steps, coefficients once per two steps, halos), against 66
@@ -137,59 +143,45 @@ struct TbTermBuf {
   TbTermRef t[2][kTbTermCap];
 };
 
-// One level of the two-step pass for one thread's z pair: the step from the
-// plane whose centre pair is at `P + o` (row stride `RS`, component stride
-// `CS`), with the plane after it at `Pn` and the centre values of the plane
-// before it in (pu, pd).  Writes the new u and the increment of each
-// component to `out + c * ocs` and `out + (3 + c) * ocs` (inactive cells:
-// 0) and, when `snap` is set, the new u of active cells to snap[3 c'] of the
-// AoS snapshot.  (pu, pd) become this plane's centres.  The switches are
-// template arguments fixed per tile: viscosity, damping, whether the pair of
-// steps adds force terms, whether it writes a snapshot.
-template <bool VISC, bool DAMP, bool PUSH, bool SNAP, int RS, int CS>
-__device__ __forceinline__ void tb_pair_step(const float* __restrict__ P,
-                                             const float* __restrict__ Pn, int o, float2 M,
-                                             float2 E, float2 (&pu)[3], float2 (&pd)[3],
-                                             bool act_a, bool act_b, const Lap7Pair& lk,
-                                             float damp, const TbTermRef* __restrict__ terms,
-                                             int nterms, unsigned nc, long long i, long long pf,
-                                             float* __restrict__ out, unsigned ocs,
-                                             float* __restrict__ snap) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const int oc = o + c * CS, od = oc + 3 * CS;
-    const float2 C = tb_ld2(P + oc), L = tb_ld2(P + oc - 2), R = tb_ld2(P + oc + 2);
-    const float2 N = tb_ld2(P + oc + RS), S = tb_ld2(P + oc - RS), X = tb_ld2(Pn + oc);
-    const float2 lu = lap7_pair(C, L, R, X, pu[c], N, S, lk);
-    const float2 Cd = tb_ld2(P + od);
-    float2 inc = ffma2(M, lu, Cd);
-    if (VISC) {
-      const float2 Ld = tb_ld2(P + od - 2), Rd = tb_ld2(P + od + 2);
-      const float2 Nd = tb_ld2(P + od + RS), Sd = tb_ld2(P + od - RS), Xd = tb_ld2(Pn + od);
-      inc = ffma2(E, lap7_pair(Cd, Ld, Rd, Xd, pd[c], Nd, Sd, lk), inc);
-      pd[c] = Cd;
-    }
-    pu[c] = C;
-    if (PUSH) {
-      for (int j = 0; j < nterms; ++j) {
-        const TbTermRef r = terms[j];
-        const float* pp = r.base + (long long)c * nc + i;
-        // the pattern is read with plain loads, outside the TMA ring: ask L2
-        // for the next plane's now (pf: its offset, 0 when there is none)
-        if (pf != 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(pp + pf));
-        const float2 Pt = __ldg(reinterpret_cast<const float2*>(pp));
-        inc = ffma2(Pt, splat2(r.scale), inc);
-      }
-    }
-    if (DAMP) inc = fmul2(inc, splat2(damp));
-    const float2 un = fadd2(C, inc);
-    tb_st2(out + (size_t)c * ocs, act_a ? un.x : 0.f, act_b ? un.y : 0.f);
-    tb_st2(out + (size_t)(3 + c) * ocs, act_a ? inc.x : 0.f, act_b ? inc.y : 0.f);
-    if (SNAP && snap != nullptr) {
-      if (act_a) snap[c] = un.x;
-      if (act_b) snap[3 + c] = un.y;
+// The z neighbours of a pair come from the lanes either side: (left's .y,
+// right's .x).  The first and last lane of a row get a value of another row
+// (or their own) in the half that looks outside the region, which no cell
+// that is used depends on: level 1 needs only the inner cell of the region's
+// outermost pairs, and level 2 leaves those pairs out.
+__device__ __forceinline__ float2 tb_zsum(float2 C) {
+  const float l = __shfl_up_sync(0xffffffffu, C.y, 1);
+  const float r = __shfl_down_sync(0xffffffffu, C.x, 1);
+  return make_float2(__fadd_rn(C.y, l), __fadd_rn(r, C.x));
+}
+
+// New u and increment of one component of a z pair: C / Cd the pair's u and
+// d, X / Xd and Xm / Xmd those of the planes after and before, (N, S) and
+// (Nd, Sd) the rows either side, P the force increment's terms.
+template <bool VISC, bool DAMP, bool PUSH>
+__device__ __forceinline__ float2 tb_inc(float2 C, float2 Cd, float2 X, float2 Xd, float2 Xm,
+                                         float2 Xmd, float2 N, float2 S, float2 Nd, float2 Sd,
+                                         float2 M, float2 E, const Lap7Pair& lk, float damp,
+                                         const TbTermRef* __restrict__ terms, int nterms,
+                                         long long i, long long pf) {
+  const float2 lu = lap7f2(fadd2(X, Xm), fadd2(N, S), tb_zsum(C), C, lk);
+  float2 inc = ffma2(M, lu, Cd);
+  if (VISC) {
+    const float2 ld = lap7f2(fadd2(Xd, Xmd), fadd2(Nd, Sd), tb_zsum(Cd), Cd, lk);
+    inc = ffma2(E, ld, inc);
+  }
+  if (PUSH) {
+    for (int j = 0; j < nterms; ++j) {
+      const TbTermRef r = terms[j];
+      const float* pp = r.base + i;
+      // the pattern is read with plain loads, outside the TMA ring: ask L2
+      // for the next plane's now (pf: its offset, 0 when there is none)
+      if (pf != 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(pp + pf));
+      const float2 Pt = __ldg(reinterpret_cast<const float2*>(pp));
+      inc = ffma2(Pt, splat2(r.scale), inc);
     }
   }
+  if (DAMP) inc = fmul2(inc, splat2(damp));
+  return inc;
 }
 
 // Where the two-step kernel's rings and barriers live.
@@ -199,7 +191,6 @@ struct TbRings {
   float* ringL;
   WsHeader* hd;
   uint64_t* Lfull;
-  uint64_t* Lempty;
   volatile int* abort_flag;
   const TbTermBuf* terms;  // the two term buffers
 };
@@ -208,8 +199,11 @@ struct TbRings {
 // planes, level-1 slots), and whether its waits have all succeeded.
 struct TbPos {
   RingPos<TmaF32TB::NA> ca;
-  RingPos<TmaF32TB::NB> cb;
+  RingPos<TmaF32TB::NB> cb;  // filled with ring A's next plane: no barrier of its own
   RingPos<TmaF32TB::NL> lw;
+  // the level-1 slot before it (a wait on the slot before the very first
+  // plane returns at once: parity 1 of a fresh barrier)
+  RingPos<TmaF32TB::NL> lp{TmaF32TB::NL - 1, 1u};
   int ord = 0;  // tiles this warp has finished (picks the term buffer)
   bool ok = true;
 };
@@ -246,7 +240,9 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
   // level 2: rows 1..OY and pairs 1..PAIRS-2 are the output tile
   const bool out_rc = r >= 1 && r <= S::OY && pl >= 1 && pl <= S::PAIRS - 2;
   const bool store = out_rc && yin && zp < g.pz;  // pz is even: the pair is in the row
+  const bool warp_out = __any_sync(0xffffffffu, store);
   const int o = (r + 1) * W + 2 + 2 * pl, ob = r * WB + 2 + 2 * pl, ol = r * LZ + 2 * pl;
+  const int ol2 = min(max(r, 1), S::OY) * LZ + 2 * pl;  // rows 0 and OY+1 read no neighbour rows
   // the force terms of steps lit (level 1) and lit+1 (level 2)
   const TbTermBuf& tbuf = k.terms[p.ord & 1];
   const int n1 = PUSH ? tbuf.n[0] : 0;
@@ -255,16 +251,21 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
   const bool snap2 = SNAP && ((lit + 2) % in->snap_stride) == 0;
   const int slot1 = snap1 ? (lit + 1) / in->snap_stride - 1 : 0;
   const int slot2 = snap2 ? (lit + 2) / in->snap_stride - 1 : 0;
-  float2 pu[3], pd[3];  // level-0 centres of the plane before
-  float2 qu[3], qd[3];  // level-1 centres of the plane before
-  float2 Mp = make_float2(0.f, 0.f), Ep = Mp;  // coefficients of the previous plane
+  // Each thread walks its own column in registers: level 0 of planes q-1 and
+  // q, level 1 of planes q-2 and q-1 (u and d of three components).  Shared
+  // memory is read only for what other threads hold: the rows either side at
+  // both levels, and the column's next level-0 plane.
+  float2 au[3], ad[3], bu[3], bd[3];  // level 0: planes q-1, q
+  float2 eu[3], ed[3], fu[3], fd[3];  // level 1: planes q-2, q-1
+  const float2 zero2 = make_float2(0.f, 0.f);
+  float2 Mp = zero2, Ep = zero2;  // coefficients of the previous plane
   {
-    const float* P0 = k.ringA + p.ca.s * AF;
+    const float* P0 = k.ringA + p.ca.s * AF + o;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      pu[c] = tb_ld2(P0 + o + c * H * W);
-      pd[c] = VISC ? tb_ld2(P0 + o + (3 + c) * H * W) : make_float2(0.f, 0.f);
-      qu[c] = qd[c] = make_float2(0.f, 0.f);
+      au[c] = tb_ld2(P0 + c * H * W);
+      ad[c] = VISC ? tb_ld2(P0 + (3 + c) * H * W) : zero2;
+      eu[c] = ed[c] = fu[c] = fd[c] = zero2;
     }
   }
   __syncwarp();
@@ -272,11 +273,18 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
   p.ca.next();
   RingPos<T::NA> cur = p.ca;  // plane q
   if (!ws_wait(&k.hd->fullA[cur.s], cur.ph, k.abort_flag)) {
-      p.ok = false;
-      return p;
-    }
+    p.ok = false;
+    return p;
+  }
   p.ca.next();
-  RingPos<T::NL> lprev = p.lw;  // slot of level-1 plane q-1 (meaningful from q = x0)
+  {
+    const float* P0 = k.ringA + cur.s * AF + o;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      bu[c] = tb_ld2(P0 + c * H * W);
+      bd[c] = tb_ld2(P0 + (3 + c) * H * W);
+    }
+  }
   for (int q = tc.x0 - 1; q <= tc.x1; ++q) {
     const RingPos<T::NA> nxt = p.ca;  // plane q+1
     if (!ws_wait(&k.hd->fullA[nxt.s], nxt.ph, k.abort_flag)) {
@@ -284,36 +292,29 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
       return p;
     }
     p.ca.next();
-    const RingPos<T::NB> pt = p.cb;
-    if (!ws_wait(&k.hd->fullB[pt.s], pt.ph, k.abort_flag)) {
-      p.ok = false;
-      return p;
-    }
-    p.cb.next();
-    // the slot is free once every warp has read what it held before
-    if (!ws_wait(&k.Lempty[p.lw.s], p.lw.ph ^ 1u, k.abort_flag)) {
-      p.ok = false;
-      return p;
-    }
-    float* Lw = k.ringL + p.lw.s * LF;
+    float* Lw = k.ringL + p.lw.s * LF + ol;
     // ---- level 1: step lit+1 at plane q on the level-1 region ----
-    const float* Bm = k.ringB + pt.s * BF;
+    const float* Bm = k.ringB + p.cb.s * BF;
+    p.cb.next();
     const float2 Mc = tb_ld2(Bm + ob);
-    const float2 Ec = VISC ? tb_ld2(Bm + HB * WB + ob) : make_float2(0.f, 0.f);
+    const float2 Ec = VISC ? tb_ld2(Bm + HB * WB + ob) : zero2;
     const bool xin = q >= 1 && q <= g.nx - 2;
+    const float* P = k.ringA + cur.s * AF + o;
+    const float* Pn = k.ringA + nxt.s * AF + o;
+    float2 nu[3], nd[3];  // level 1 of plane q
     if (!(xin && warp_live)) {
       // every cell of the warp's rows is outside the interior: level 1 is the
-      // zero shell; keep this plane's level-0 centres for the next plane
-      const float* P = k.ringA + cur.s * AF;
+      // zero shell
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        pu[c] = tb_ld2(P + o + c * H * W);
-        if (VISC) pd[c] = tb_ld2(P + o + (3 + c) * H * W);
-        tb_st2(Lw + ol + c * LP, 0.f, 0.f);
-        tb_st2(Lw + ol + (3 + c) * LP, 0.f, 0.f);
+        nu[c] = nd[c] = zero2;
+        au[c] = bu[c];
+        bu[c] = tb_ld2(Pn + c * H * W);
+        if (VISC) ad[c] = bd[c];
+        bd[c] = tb_ld2(Pn + (3 + c) * H * W);
       }
     } else {
-      const bool aa = xin && yin && zin_a, ab = xin && yin && zin_b;
+      const bool aa = yin && zin_a, ab = yin && zin_b;
       long long i = 0;  // the pair's cell, for the force patterns
       int nl = 0;
       if (PUSH) {
@@ -324,57 +325,87 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
       float* sp = nullptr;
       if (SNAP && snap1 && store && q >= tc.x0 && q < tc.x1)
         sp = in->snaps + ((((long long)slot1 * g.nx + q) * g.ny + y) * g.nz + zp) * 3;
-      tb_pair_step<VISC, DAMP, PUSH, SNAP, W, H * W>(
-          k.ringA + cur.s * AF, k.ringA + nxt.s * AF, o, Mc, Ec, pu, pd, aa, ab, lk, damp,
-          tbuf.t[0], nl, nc, i, PUSH && q + 1 <= g.nx - 2 ? g.sxy : 0, Lw + ol, (unsigned)LP,
-          sp);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float* Pc = P + c * H * W;
+        const float* Pd = P + (3 + c) * H * W;
+        const float2 X = tb_ld2(Pn + c * H * W), Xd = tb_ld2(Pn + (3 + c) * H * W);
+        const float2 inc = tb_inc<VISC, DAMP, PUSH>(
+            bu[c], bd[c], X, Xd, au[c], ad[c], tb_ld2(Pc + W), tb_ld2(Pc - W),
+            VISC ? tb_ld2(Pd + W) : zero2, VISC ? tb_ld2(Pd - W) : zero2, Mc, Ec, lk, damp,
+            tbuf.t[0], nl, c * (long long)nc + i, PUSH && q + 1 <= g.nx - 2 ? g.sxy : 0);
+        const float2 un = fadd2(bu[c], inc);
+        nu[c] = make_float2(aa ? un.x : 0.f, ab ? un.y : 0.f);
+        nd[c] = make_float2(aa ? inc.x : 0.f, ab ? inc.y : 0.f);
+        if (SNAP && sp != nullptr) {
+          if (aa) sp[c] = un.x;
+          if (ab) sp[3 + c] = un.y;
+        }
+        au[c] = bu[c];
+        bu[c] = X;
+        if (VISC) ad[c] = bd[c];
+        bd[c] = Xd;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      tb_st2(Lw + c * LP, nu[c].x, nu[c].y);
+      tb_st2(Lw + (3 + c) * LP, nd[c].x, nd[c].y);
     }
     __syncwarp();
     if (lane == 0) {
       mbar_arrive(&k.hd->emptyA[cur.s]);  // level-0 plane q is no longer needed
-      mbar_arrive(&k.hd->emptyB[pt.s]);
       mbar_arrive(&k.Lfull[p.lw.s]);      // this warp's row of level-1 plane q is written
     }
-    if (q >= tc.x0) {
-      const float* Lc = k.ringL + lprev.s * LF;  // level-1 plane q-1
-      if (q == tc.x0) {  // level-1 centres of plane x0-1 (own pair) for the first level 2
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          qu[c] = tb_ld2(Lc + ol + c * LP);
-          qd[c] = VISC ? tb_ld2(Lc + ol + (3 + c) * LP) : make_float2(0.f, 0.f);
-        }
-      } else {
-        // ---- level 2: step lit+2 at plane x = q-1 on the output tile ----
-        // (reads rows r-1..r+1 of plane q-1: wait until every warp wrote it)
-        if (!ws_wait(&k.Lfull[lprev.s], lprev.ph, k.abort_flag)) {
+    // every warp has written plane q-1 (and has left iteration q-2, so the
+    // slot after the next, plane q-3's, can be written again)
+    if (!ws_wait(&k.Lfull[p.lp.s], p.lp.ph, k.abort_flag)) {
       p.ok = false;
       return p;
     }
+    if (q > tc.x0 && warp_out) {
+      // ---- level 2: step lit+2 at plane x = q-1 on the output tile ----
+      const float* Lc = k.ringL + p.lp.s * LF + ol2;  // a row of the output tile
+      const int x = q - 1;
+      const long long i = (long long)x * g.sxy + (long long)y * g.pz + zp;
+      float* sp = nullptr;
+      if (SNAP && snap2 && store)
+        sp = in->snaps + ((((long long)slot2 * g.nx + x) * g.ny + y) * g.nz + zp) * 3;
+      float* out = D + i;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float* Pc = Lc + c * LP;
+        const float* Pd = Lc + (3 + c) * LP;
+        const float2 inc = tb_inc<VISC, DAMP, PUSH>(
+            fu[c], fd[c], nu[c], nd[c], eu[c], ed[c], tb_ld2(Pc + LZ), tb_ld2(Pc - LZ),
+            VISC ? tb_ld2(Pd + LZ) : zero2, VISC ? tb_ld2(Pd - LZ) : zero2, Mp, Ep, lk, damp,
+            tbuf.t[1], PUSH && store ? n2 : 0, c * (long long)nc + i, 0);
+        const float2 un = fadd2(fu[c], inc);
         if (store) {
-          const int x = q - 1;
-          const long long i = (long long)x * g.sxy + (long long)y * g.pz + zp;
-          float* sp = nullptr;
-          if (SNAP && snap2)
-            sp = in->snaps + ((((long long)slot2 * g.nx + x) * g.ny + y) * g.nz + zp) * 3;
-          tb_pair_step<VISC, DAMP, PUSH, SNAP, LZ, LP>(Lc, Lw, ol, Mp, Ep, qu, qd, zin_a, zin_b,
-                                                       lk, damp, tbuf.t[1], n2, nc, i, 0, D + i,
-                                                       nc, sp);
+          tb_st2(out + (size_t)c * nc, zin_a ? un.x : 0.f, zin_b ? un.y : 0.f);
+          tb_st2(out + (size_t)(3 + c) * nc, zin_a ? inc.x : 0.f, zin_b ? inc.y : 0.f);
+        }
+        if (SNAP && sp != nullptr) {
+          if (zin_a) sp[c] = un.x;
+          if (zin_b) sp[3 + c] = un.y;
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&k.Lempty[lprev.s]);  // this warp is done with plane q-1
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      eu[c] = fu[c];
+      fu[c] = nu[c];
+      if (VISC) ed[c] = fd[c];
+      fd[c] = nd[c];
     }
     Mp = Mc;
     Ep = Ec;
-    lprev = p.lw;
+    p.lp = p.lw;
     p.lw.next();
     cur = nxt;
   }
   __syncwarp();
-  if (lane == 0) {
-    mbar_arrive(&k.hd->emptyA[cur.s]);  // the closing halo plane x1+1
-    mbar_arrive(&k.Lempty[lprev.s]);    // the tile's last level-1 plane x1
-  }
+  if (lane == 0) mbar_arrive(&k.hd->emptyA[cur.s]);  // the closing halo plane x1+1
   return p;
 }
 
@@ -445,8 +476,7 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
   float* ringB = ringA + NA * AF;
   float* ringL = ringB + NB * BF;
   uint64_t* Lfull = reinterpret_cast<uint64_t*>(ringL + NL * LF);  // after the rings
-  uint64_t* Lempty = Lfull + NL;
-  TbTermBuf* terms = reinterpret_cast<TbTermBuf*>(Lempty + NL);
+  TbTermBuf* terms = reinterpret_cast<TbTermBuf*>(Lfull + NL);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   auto flags_of = [&](int k) -> int* { return BATCH ? tab[k].flags : one.flags; };
   if ((smem_addr(ringA) & 127u) != 0u) {
@@ -462,14 +492,7 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
       mbar_init(&hd->fullA[s], 1);
       mbar_init(&hd->emptyA[s], T::CONSUMER_WARPS);
     }
-    for (int s = 0; s < NB; ++s) {
-      mbar_init(&hd->fullB[s], 1);
-      mbar_init(&hd->emptyB[s], T::CONSUMER_WARPS);
-    }
-    for (int s = 0; s < NL; ++s) {
-      mbar_init(&Lfull[s], T::CONSUMER_WARPS);
-      mbar_init(&Lempty[s], T::CONSUMER_WARPS);
-    }
+    for (int s = 0; s < NL; ++s) mbar_init(&Lfull[s], T::CONSUMER_WARPS);
     *abort_flag = 0;
     abort_flag[1] = BATCH ? (ninst > 0 ? tab[0].wait_k : 1) : one.wait_k;
     lg->n_taken = 0;
@@ -515,7 +538,9 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
         const CUtensorMap* tma = &in->tm[lit % 3];
         const uint32_t bbytes = dm.b_cells * 4 * in->ncoef;
         bool first = true;
-        auto issueA = [&](int p) {
+        // level-0 plane p, and from plane x0 on the coefficients of plane p-1
+        // (what level 1 of plane p-1 reads) on the same barrier
+        auto issue = [&](int p) {
           const int sa = pa.s;
           ok = ok && ws_wait(&hd->emptyA[sa], pa.ph ^ 1u, abort_flag);
           if (!ok) return;
@@ -541,33 +566,23 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
           }
           const int pl = min(max(p, 0), g.nx - 1);  // planes outside the grid feed only the shell
           fence_proxy_async_smem();
-          mbar_arrive_expect_tx(&hd->fullA[sa], dm.a_bytes);
+          const bool points = p >= tc.x0;
+          mbar_arrive_expect_tx(&hd->fullA[sa], dm.a_bytes + (points ? bbytes : 0u));
           tma_load_4d(ringA + sa * AF, tma, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 2, pl, 0);
+          if (points) {
+            const int ql = min(max(p - 1, 0), g.nx - 1);
+            tma_load_4d(ringB + pb.s * BF, &in->tmm, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 1, ql, 0);
+            pb.next();
+          }
           arm_record(lg->armedA, lg->parA, sa, pa.ph);
           pa.next();
         };
-        auto issueB = [&](int q) {
-          const int sb = pb.s;
-          ok = ok && ws_wait(&hd->emptyB[sb], pb.ph ^ 1u, abort_flag);
-          if (!ok) return;
-          const int ql = min(max(q, 0), g.nx - 1);
-          fence_proxy_async_smem();
-          mbar_arrive_expect_tx(&hd->fullB[sb], bbytes);
-          tma_load_4d(ringB + sb * BF, &in->tmm, &hd->fullB[sb], tc.z0 - 4, tc.y0 - 1, ql, 0);
-          arm_record(lg->armedB, lg->parB, sb, pb.ph);
-          pb.next();
-        };
-        issueA(tc.x0 - 2);
-        issueA(tc.x0 - 1);
-        for (int q = tc.x0 - 1; q <= tc.x1 && ok; ++q) {
-          issueA(q + 1);
-          issueB(q);
-        }
+        for (int p = tc.x0 - 2; p <= tc.x1 + 1 && ok; ++p) issue(p);
       }
     }
   } else {
     // ------------------------------- consumers ----------------------------
-    const TbRings k{ringA, ringB, ringL, hd, Lfull, Lempty, abort_flag, terms};
+    const TbRings k{ringA, ringB, ringL, hd, Lfull, abort_flag, terms};
     TbPos p;
     while (true) {
       // the tile's first plane, x0-2: centres only
@@ -591,7 +606,6 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
   if (*abort_flag && warp == T::CONSUMER_WARPS && lane == 0) {
     // let every copy still in flight land, then flag the abandoned tiles' solves
     drain_ring(hd->fullA, lg->armedA, lg->parA, NA);
-    drain_ring(hd->fullB, lg->armedB, lg->parB, NB);
     flag_unfinished(lg, T::CONSUMER_WARPS, BATCH ? ninst : 1, kFlagTimeout, flags_of);
   }
   queue_cta_done(queue);
@@ -602,12 +616,12 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// alignment slack + header + rings + the level-1 ring's full / empty barriers
-// + the two term buffers
+// alignment slack + header + rings + the level-1 ring's barriers + the two
+// term buffers
 size_t tb_smem_bytes() {
   return 128 + kRingOffset + (size_t)TmaF32TB::NA * TmaF32TB::A_STAGE +
          (size_t)TmaF32TB::NB * TmaF32TB::B_STAGE + (size_t)TmaF32TB::NL * TmaF32TB::L_STAGE +
-         2 * TmaF32TB::NL * sizeof(uint64_t) + 2 * sizeof(TbTermBuf);
+         TmaF32TB::NL * sizeof(uint64_t) + 2 * sizeof(TbTermBuf);
 }
 
 static int tb_set_attr() {
