@@ -68,154 +68,333 @@ __host__ __device__ inline double basis_entry(int n, double h, int row, int col,
   return sqrt(2.0 / (K + 0.5)) * cos((jj + 0.5) * (k + 0.5) * M_PI / (K + 0.5));
 }
 
-// The solve builds its bases on the device, one thread per entry (the host
-// would spend ~1 ms per solve on the m^2 cosines, with the GPU waiting).
-__global__ void axis_basis_kernel(int n, double h, double* __restrict__ Q,
-                                  double* __restrict__ lam) {
-  const int m = n - 2;
+// One axis of the solve: its two chains (0: even grid indices, 1: odd ones),
+// chain position j at grid index first + 2 j.  Mode k of a chain is stored at
+// the grid index of position k, so every transform has one form,
+//     out[first + 2 a] = sum_b W[b][a] in[first + 2 b],
+// with W = Q forward and Q^T back (both K x K, row-major).
+struct AxisBasis {
+  double* W[2][2];  // [forward 0 / inverse 1][chain]
+  double* lam;      // eigenvalue of the mode at grid index i, at i - 1
+  int K[2];
+};
+__host__ __device__ inline int chain_first(int par) { return par == 0 ? 2 : 1; }
+__host__ __device__ inline int chain_len(int n, int par) {
+  const int first = chain_first(par);
+  return first > n - 2 ? 0 : (n - 2 - first) / 2 + 1;
+}
+
+// The solve builds its bases on the device, one thread per entry of the two
+// chains' matrices (the host would spend ~1 ms per solve on the cosines, with
+// the GPU waiting).
+__global__ void axis_basis_kernel(int n, double h, AxisBasis ax) {
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (m <= 0 || e >= (long long)m * m) return;
-  const int row = (int)(e / m), col = (int)(e % m);
-  Q[e] = basis_entry(n, h, row, col, row == 0 ? lam + col : nullptr);
+  const long long n0 = (long long)ax.K[0] * ax.K[0];
+  const int par = e < n0 ? 0 : 1;
+  const long long q = par ? e - n0 : e;
+  const int K = ax.K[par];
+  if (q >= (long long)K * K) return;
+  const int j = (int)(q / K), k = (int)(q % K);
+  const int row = chain_first(par) + 2 * j - 1;  // interior index of the position
+  const int col = par ? ax.K[0] + k : k;
+  double lam;
+  const double v = basis_entry(n, h, row, col, j == 0 ? &lam : nullptr);
+  ax.W[0][par][(long long)j * K + k] = v;
+  ax.W[1][par][(long long)k * K + j] = v;
+  if (j == 0) ax.lam[chain_first(par) + 2 * k - 1] = lam;
 }
 
 // ---------------------------------------------------------------------------
-// strided batched FP64 GEMM: C = A B
+// one-axis transforms in FP64
 // ---------------------------------------------------------------------------
-struct Mat {
-  const double* p;
-  long long rs, cs, bs;  // row, column and batch strides (elements)
-};
+// A basis couples cells of one parity only, so an axis of n cells is two
+// products with matrices of n/2 rows: half the multiply-adds of one n x n
+// product.  What bounds them is the FP64 pipe (64 fused multiply-adds per
+// cycle and SM).  A warp owns 32 modes x 32 data columns, a thread 8 x 4
+// accumulators (six to eight shared-memory wavefronts per 32 multiply-adds
+// of the warp, under half of what the pipe leaves time for), operands come
+// through a three-stage cp.async ring 16 deep.  A block takes WM units of 32
+// modes: a chain of up to 128 modes reads its data once and pads its modes
+// to a multiple of 32 only.  Measured against 64 x 64 tiles of the full
+// n x n matrices with 8-byte loads and no pipeline: the six transforms of a
+// 160 x 131 x 173 grid 1154 -> 339 us (whole projection 1406 -> 523 us), the
+// 48 of eight 256 x 256 x 384 forces 75.4 -> 21.0 ms (axes x and y at 20
+// TFLOP/s of the multiply-adds a chain needs, axis z at 14.5).
+constexpr int SG_K = 16, SG_STAGES = 3;
 
-constexpr int GB_M = 64, GB_N = 64, GB_K = 16;
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(ok ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(ok ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
-__global__ void __launch_bounds__(256) gemm_f64(Mat A, Mat B, double* C, long long crs,
-                                                long long ccs, long long cbs, int M, int N,
-                                                int K) {
-  __shared__ double As[GB_K][GB_M + 1];
-  __shared__ double Bs[GB_K][GB_N + 1];
-  const int b = blockIdx.z;
-  const double* Ab = A.p + b * A.bs;
-  const double* Bb = B.p + b * B.bs;
-  double* Cb = C + b * cbs;
-  const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GB_N;
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  double acc[4][4] = {};
-  const bool a_rowmajor = (A.cs == 1);
-  const bool b_rowmajor = (B.cs == 1);
-  for (int k0 = 0; k0 < K; k0 += GB_K) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int e = t + 256 * q;
-      int r, c;  // A tile element (r in M, c in K)
-      if (a_rowmajor) {
-        r = e / GB_K;
-        c = e % GB_K;
-      } else {
-        r = e % GB_M;
-        c = e / GB_M;
-      }
-      const int gr = m0 + r, gc = k0 + c;
-      As[c][r] = (gr < M && gc < K) ? Ab[gr * A.rs + gc * A.cs] : 0.0;
-      int rb, cb;  // B tile element (rb in K, cb in N)
-      if (b_rowmajor) {
-        rb = e / GB_N;
-        cb = e % GB_N;
-      } else {
-        rb = e % GB_K;
-        cb = e / GB_K;
-      }
-      const int gk = k0 + rb, gn = n0 + cb;
-      Bs[rb][cb] = (gk < K && gn < N) ? Bb[gk * B.rs + gn * B.cs] : 0.0;
+// Rows b0 .. b0+15 of a chain's matrix, columns a0 .. a0+32 WM-1 (zero
+// outside the matrix).
+template <int WM, int THREADS>
+__device__ __forceinline__ void load_w(double* __restrict__ ws, const double* __restrict__ W,
+                                       int K, int b0, int a0, int tid) {
+  constexpr int LD = 32 * WM;
+  for (int e = tid; e < SG_K * LD; e += THREADS) {
+    const int kk = e / LD, a = e % LD;
+    const int b = b0 + kk, col = a0 + a;
+    const bool ok = b >= 0 && b < K && col < K;
+    cp_async8(ws + kk * LD + a, ok ? W + (long long)b * K + col : W, ok);
+  }
+}
+
+// Axes x and y: rows of the padded field are `rs` apart; the data columns are
+// numbered n, `nper` of them contiguous and then `nstride` on (axis x: one
+// run of a whole plane; axis y: the z rows of all interior planes).  nper is
+// even, so the 16-byte pieces never straddle two runs.
+template <int WM>
+__global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
+    spec_rows(AxisBasis ax, int inverse, const double* __restrict__ src, double* __restrict__ dst,
+              long long rs, int nper, long long nstride, long long ntot) {
+  constexpr int THREADS = 64 * WM, LDW = 32 * WM, LDD = 64;
+  extern __shared__ __align__(16) double smem[];
+  double* wsm = smem;                               // [stage][16][32 WM]
+  double* dsm = smem + SG_STAGES * SG_K * LDW;      // [stage][16][64]
+  const int par = blockIdx.z, K = ax.K[par];
+  const int a0 = blockIdx.y * LDW;
+  if (a0 >= K) return;
+  const double* W = ax.W[inverse][par];
+  const long long n0 = blockIdx.x * 64ll;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wm = warp % WM, wn = warp / WM, gm = lane >> 3, gn = lane & 7;
+  const double* base = src + chain_first(par) * rs;
+  // pieces of two columns: this thread copies piece tid % 32 of some rows
+  const long long pn = n0 + 2 * (tid & 31);
+  const bool pok = pn < ntot;
+  const long long poff = pok ? (pn / nper) * nstride + pn % nper : 0;
+  auto load = [&](int st, int b0) {
+    load_w<WM, THREADS>(wsm + st * SG_K * LDW, W, K, b0, a0, tid);
+    for (int kk = tid >> 5; kk < SG_K; kk += THREADS / 32) {
+      const bool ok = pok && b0 + kk < K;
+      cp_async16(dsm + (st * SG_K + kk) * LDD + 2 * (tid & 31),
+                 ok ? base + 2 * (b0 + kk) * rs + poff : src, ok);
     }
+  };
+  double acc[8][4] = {};
+  const int nk = (K + SG_K - 1) / SG_K;
+#pragma unroll
+  for (int st = 0; st < SG_STAGES - 1; ++st) {
+    if (st < nk) load(st, st * SG_K);
+    cp_async_commit();
+  }
+  for (int c = 0; c < nk; ++c) {
+    cp_async_wait<SG_STAGES - 2>();
     __syncthreads();
+    const int nx = c + SG_STAGES - 1;
+    if (nx < nk) load(nx % SG_STAGES, nx * SG_K);
+    cp_async_commit();
+    const double* wp = wsm + (c % SG_STAGES) * SG_K * LDW + wm * 32 + 2 * gm;
+    const double* dp = dsm + (c % SG_STAGES) * SG_K * LDD + wn * 32 + 2 * gn;
+#pragma unroll 4
+    for (int kk = 0; kk < SG_K; ++kk) {
+      double2 w[4], d[2];
 #pragma unroll
-    for (int kk = 0; kk < GB_K; ++kk) {
-      double a[4], bb[4];
+      for (int i = 0; i < 4; ++i)
+        w[i] = *reinterpret_cast<const double2*>(wp + kk * LDW + 8 * i);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) bb[j] = Bs[kk][tx * 4 + j];
+      for (int j = 0; j < 2; ++j)
+        d[j] = *reinterpret_cast<const double2*>(dp + kk * LDD + 16 * j);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], bb[j], acc[i][j]);
+        for (int j = 0; j < 2; ++j) {
+          acc[2 * i][2 * j] = fma(w[i].x, d[j].x, acc[2 * i][2 * j]);
+          acc[2 * i][2 * j + 1] = fma(w[i].x, d[j].y, acc[2 * i][2 * j + 1]);
+          acc[2 * i + 1][2 * j] = fma(w[i].y, d[j].x, acc[2 * i + 1][2 * j]);
+          acc[2 * i + 1][2 * j + 1] = fma(w[i].y, d[j].y, acc[2 * i + 1][2 * j + 1]);
+        }
     }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const long long n = n0 + wn * 32 + 16 * j + 2 * gn;
+    if (n >= ntot) continue;
+    double* out = dst + (n / nper) * nstride + n % nper;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int a = a0 + wm * 32 + 8 * (i >> 1) + 2 * gm + (i & 1);
+      if (a < K)
+        *reinterpret_cast<double2*>(out + (chain_first(par) + 2ll * a) * rs) =
+            make_double2(acc[i][2 * j], acc[i][2 * j + 1]);
+    }
+  }
+}
+
+// Axis z: 32 lines (x, y) per block, both chains (the two halves of its
+// warps), so each line is read and written in whole rows; the results pass
+// through shared memory to leave in row order.  Lines are the interior
+// (x, y).  With `scale` the results are divided by the eigenvalue sums (zero
+// on the null modes), which ends the forward transforms.
+template <int WM>
+__global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
+    spec_lines(AxisBasis ax, int inverse, const double* __restrict__ src,
+               double* __restrict__ dst, Geom g, int scale, const double* __restrict__ lx,
+               const double* __restrict__ ly, double lam_floor) {
+  constexpr int THREADS = 64 * WM, LDW = 32 * WM, LDD = 2 * SG_K + 2, LDE = 64 * WM + 1;
+  extern __shared__ __align__(16) double smem[];
+  double* wsm = smem;                                // [stage][chain][16][32 WM]
+  double* dsm = smem + SG_STAGES * 2 * SG_K * LDW;   // [stage][32 lines][34]
+  __shared__ long long loff[32];
+  __shared__ double lsum[32];
+  const int a0 = blockIdx.y * LDW;
+  const long long l0 = blockIdx.x * 32ll, nl = (long long)(g.nx - 2) * (g.ny - 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int par = warp / WM, wm = warp % WM, gm = lane >> 3, gn = lane & 7;
+  if (tid < 32) {
+    const long long l = l0 + tid;
+    const int x = (int)(l / (g.ny - 2)) + 1, y = (int)(l % (g.ny - 2)) + 1;
+    loff[tid] = l < nl ? x * g.sxy + (long long)y * g.pz : -1;
+    lsum[tid] = scale && l < nl ? lx[x - 1] + ly[y - 1] : 0.0;
+  }
+  __syncthreads();
+  // 16-byte pieces: 16 per line, THREADS / 16 lines at a time
+  auto load = [&](int st, int c) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p)  // z = 32 c + 2 t: even chain position 16 c + t - 1
+      load_w<WM, THREADS>(wsm + (st * 2 + p) * SG_K * LDW, ax.W[inverse][p], ax.K[p],
+                          c * SG_K - (p == 0 ? 1 : 0), a0, tid);
+    const int z = 2 * SG_K * c + 2 * (tid & 15);
+    for (int l = tid >> 4; l < 32; l += THREADS / 16) {
+      const bool ok = loff[l] >= 0 && z < g.pz;
+      cp_async16(dsm + (st * 32 + l) * LDD + 2 * (tid & 15), ok ? src + loff[l] + z : src, ok);
+    }
+  };
+  double acc[8][4] = {};
+  const int nk = (g.nz - 1 + 2 * SG_K - 1) / (2 * SG_K);  // z = 0 .. nz-2
+#pragma unroll
+  for (int st = 0; st < SG_STAGES - 1; ++st) {
+    if (st < nk) load(st, st);
+    cp_async_commit();
+  }
+  for (int c = 0; c < nk; ++c) {
+    cp_async_wait<SG_STAGES - 2>();
     __syncthreads();
+    const int nx = c + SG_STAGES - 1;
+    if (nx < nk) load(nx % SG_STAGES, nx);
+    cp_async_commit();
+    const double* wp = wsm + ((c % SG_STAGES) * 2 + par) * SG_K * LDW + wm * 32 + 2 * gm;
+    const double* dp = dsm + ((c % SG_STAGES) * 32 + gn) * LDD + (par == 0 ? 0 : 1);
+#pragma unroll 4
+    for (int kk = 0; kk < SG_K; ++kk) {
+      double2 w[4];
+      double d[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        w[i] = *reinterpret_cast<const double2*>(wp + kk * LDW + 8 * i);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) d[j] = dp[8 * j * LDD + 2 * kk];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[2 * i][j] = fma(w[i].x, d[j], acc[2 * i][j]);
+          acc[2 * i + 1][j] = fma(w[i].y, d[j], acc[2 * i + 1][j]);
+        }
+    }
   }
+  cp_async_wait<0>();
+  __syncthreads();  // the ring is free: rows of results take its place
+  // odd chain's mode a at z = 1 + 2 a, even chain's at 2 + 2 a
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gr = m0 + ty * 4 + i;
-    if (gr >= M) continue;
+  for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx * 4 + j;
-      if (gn < N) Cb[gr * crs + gn * ccs] = acc[i][j];
+    for (int j = 0; j < 4; ++j)
+      smem[(gn + 8 * j) * LDE + 2 * (wm * 32 + 8 * (i >> 1) + 2 * gm + (i & 1)) +
+           (par == 0 ? 1 : 0)] = acc[i][j];
+  __syncthreads();
+  const int z0 = 1 + 2 * a0, zn = min(2 * LDW, g.nz - 2 + 1 - z0);
+  for (int l = warp; l < 32; l += THREADS / 32) {
+    if (loff[l] < 0) continue;
+    for (int r = lane; r < zn; r += 32) {
+      double v = smem[l * LDE + r];
+      if (scale) {
+        const double L = lsum[l] + ax.lam[z0 + r - 1];
+        v = L > lam_floor ? v / L : 0.0;
+      }
+      dst[loff[l] + z0 + r] = v;
     }
   }
 }
 
-// b_hat /= (lx_i + ly_j + lz_k) on interior cells; zero on the null modes
-__global__ void spectral_scale(double* v, Geom g, const double* __restrict__ lx,
-                               const double* __restrict__ ly, const double* __restrict__ lz,
-                               double lam_floor) {
-  const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(q % (g.nz - 2));
-    const long long r = q / (g.nz - 2);
-    const int j = (int)(r % (g.ny - 2));
-    const int i = (int)(r / (g.ny - 2));
-    const long long idx = (long long)(i + 1) * g.sxy + (long long)(j + 1) * g.pz + (k + 1);
-    const double L = lx[i] + ly[j] + lz[k];
-    v[idx] = (L > lam_floor) ? v[idx] / L : 0.0;
-  }
+// Units of 32 modes per block for a chain of K modes: all of them up to four,
+// else the count whose blocks pad the modes least.
+static int mode_units(int K) {
+  const int u = std::max(1, (K + 31) / 32);
+  if (u <= 4) return u;
+  int best = 4;
+  for (int w = 3; w >= 2; --w)
+    if ((u + w - 1) / w * w < (u + best - 1) / best * best) best = w;
+  return best;
 }
 
-static int launch_gemm(Mat A, Mat B, double* C, long long crs, long long ccs, long long cbs,
-                       int M, int N, int K, int batch, cudaStream_t s) {
-  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return SW_OK;
-  dim3 grid((N + GB_N - 1) / GB_N, (M + GB_M - 1) / GB_M, batch);
-  gemm_f64<<<grid, 256, 0, s>>>(A, B, C, crs, ccs, cbs, M, N, K);
+constexpr size_t spec_rows_smem(int wm) {
+  return sizeof(double) * SG_STAGES * SG_K * (32 * wm + 64);
+}
+constexpr size_t spec_lines_smem(int wm) {
+  const size_t ring = sizeof(double) * SG_STAGES * (2 * SG_K * 32 * wm + 32 * (2 * SG_K + 2));
+  const size_t rows = sizeof(double) * 32 * (64 * wm + 1);
+  return ring > rows ? ring : rows;
+}
+
+template <int WM>
+static int launch_axis(const Geom& g, int axis, const AxisBasis& ax, bool inverse,
+                       const double* src, double* dst, bool scale, const double* lx,
+                       const double* ly, double lam_floor, cudaStream_t s) {
+  const int Kmax = std::max(ax.K[0], ax.K[1]);
+  const unsigned mt = (unsigned)((Kmax + 32 * WM - 1) / (32 * WM));
+  cudaError_t e;
+  if (axis == 2) {
+    const size_t sm = spec_lines_smem(WM);
+    e = cudaFuncSetAttribute(spec_lines<WM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(spectral lines)");
+    const long long nl = (long long)(g.nx - 2) * (g.ny - 2);
+    spec_lines<WM><<<dim3((unsigned)((nl + 31) / 32), mt), 64 * WM, sm, s>>>(
+        ax, inverse ? 1 : 0, src, dst, g, scale ? 1 : 0, lx, ly, lam_floor);
+  } else {
+    const size_t sm = spec_rows_smem(WM);
+    e = cudaFuncSetAttribute(spec_rows<WM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(spectral rows)");
+    const long long ntot = axis == 0 ? g.sxy : (long long)(g.nx - 2) * g.pz;
+    const dim3 grid((unsigned)((ntot + 63) / 64), mt, 2);
+    if (axis == 0)  // all (y, z) columns of the plane
+      spec_rows<WM><<<grid, 64 * WM, sm, s>>>(ax, inverse ? 1 : 0, src, dst, g.sxy, (int)g.sxy, 0,
+                                              ntot);
+    else  // the z columns of every interior plane
+      spec_rows<WM><<<grid, 64 * WM, sm, s>>>(ax, inverse ? 1 : 0, src + g.sxy, dst + g.sxy, g.pz,
+                                              g.pz, g.sxy, ntot);
+  }
   count_launches(1);
   SW_CHECK_LAUNCH("spectral transform");
   return SW_OK;
 }
 
-// Transform along `axis` (0 x, 1 y, 2 z) of the padded field src into dst:
-// forward (dst = Q^T src) or inverse (dst = Q src) on interior indices.
-static int axis_transform(const Geom& g, int axis, const double* Q, bool forward,
-                          const double* src, double* dst, cudaStream_t s) {
-  const int nax = axis == 0 ? g.nx : (axis == 1 ? g.ny : g.nz);
-  const int m = nax - 2;
-  if (m <= 0) return SW_OK;
-  // operator as an m x m matrix: forward uses Q^T (row k, col i) = Q[i*m + k]
-  Mat Op;
-  Op.p = Q;
-  Op.bs = 0;
-  if (forward) {
-    Op.rs = 1;
-    Op.cs = m;
-  } else {
-    Op.rs = m;
-    Op.cs = 1;
+// Transform along `axis` (0 x, 1 y, 2 z) of the interior of the padded field
+// src into dst.
+static int axis_transform(const Geom& g, int axis, const AxisBasis& ax, bool inverse,
+                          const double* src, double* dst, bool scale, const double* lx,
+                          const double* ly, double lam_floor, cudaStream_t s) {
+  switch (mode_units(std::max(ax.K[0], ax.K[1]))) {
+    case 1: return launch_axis<1>(g, axis, ax, inverse, src, dst, scale, lx, ly, lam_floor, s);
+    case 2: return launch_axis<2>(g, axis, ax, inverse, src, dst, scale, lx, ly, lam_floor, s);
+    case 3: return launch_axis<3>(g, axis, ax, inverse, src, dst, scale, lx, ly, lam_floor, s);
+    default: return launch_axis<4>(g, axis, ax, inverse, src, dst, scale, lx, ly, lam_floor, s);
   }
-  if (axis == 0) {  // C[k][l] = Op[k][i] D[i+1][l], l over all (y, z)
-    Mat D{src + g.sxy, g.sxy, 1, 0};
-    return launch_gemm(Op, D, dst + g.sxy, g.sxy, 1, 0, m, (int)g.sxy, m, 1, s);
-  }
-  if (axis == 1) {  // per x plane: C[k][z] = Op[k][j] D[x][j+1][z]
-    Mat D{src + g.pz, g.pz, 1, g.sxy};
-    return launch_gemm(Op, D, dst + g.pz, g.pz, 1, g.sxy, m, g.pz, m, g.nx, s);
-  }
-  // axis z: C[l][k] = D[l][i+1] Op^T[i][k], l over all (x, y) lines
-  Mat D{src + 1, g.pz, 1, 0};
-  Mat OpT;  // (i, k) -> Op[k][i]
-  OpT.p = Q;
-  OpT.bs = 0;
-  OpT.rs = Op.cs;
-  OpT.cs = Op.rs;
-  return launch_gemm(D, OpT, dst + 1, g.pz, 1, 0, g.nx * g.ny, m, m, 1, s);
 }
 
 size_t spectral_extra_bytes(const Geom& g) {
@@ -234,63 +413,76 @@ using namespace sw;
 
 namespace {
 
+// Blocks of 32 (z) x 8 (y) threads over the padded cells, a few x planes per
+// block: no division per cell, and the shell and padding are written here
+// too, so neither the rhs nor the output is cleared beforehand.
+constexpr int kSpecPlanes = 8;
+dim3 spec_grid(const Geom& g) {
+  return dim3((unsigned)((g.pz + TILE_Z - 1) / TILE_Z), (unsigned)((g.ny + TILE_Y - 1) / TILE_Y),
+              (unsigned)((g.nx + kSpecPlanes - 1) / kSpecPlanes));
+}
+
+// rhs = -div_c(mask f) on interior cells (the CG's r0), 0 elsewhere; also max |div|
 template <typename T>
-__global__ void prep_rhs(const T* __restrict__ fx, const T* __restrict__ fy,
-                         const T* __restrict__ fz, InStride s, Geom g, double c2x, double c2y,
-                         double c2z, double* __restrict__ rhs, double* __restrict__ maxdiv) {
-  // rhs = -div_c(mask f) on interior cells (the CG's r0); also max |div|
+__global__ void __launch_bounds__(TILE_THREADS)
+    prep_rhs(const T* __restrict__ fx, const T* __restrict__ fy, const T* __restrict__ fz,
+             InStride s, Geom g, double c2x, double c2y, double c2z, double* __restrict__ rhs,
+             double* __restrict__ maxdiv) {
+  __shared__ double red[32];
   double mx = 0.0;
-  const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
   auto ld = [&](const T* f, int x, int y, int z) -> double {
     if (f == nullptr || !interior(g, x, y, z)) return 0.0;
     return (double)f[(long long)x * s.sx + (long long)y * s.sy + (long long)z * s.sz];
   };
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int z = 1 + (int)(q % (g.nz - 2));
-    const long long r = q / (g.nz - 2);
-    const int y = 1 + (int)(r % (g.ny - 2));
-    const int x = 1 + (int)(r / (g.ny - 2));
-    const double tx = (ld(fx, x + 1, y, z) - ld(fx, x - 1, y, z)) * c2x;
-    const double ty = (ld(fy, x, y + 1, z) - ld(fy, x, y - 1, z)) * c2y;
-    const double tz = (ld(fz, x, y, z + 1) - ld(fz, x, y, z - 1)) * c2z;
-    const double div = (tx + ty) + tz;
-    rhs[(long long)x * g.sxy + (long long)y * g.pz + z] = -div;
-    mx = fmax(mx, fabs(div));
+  const int z = blockIdx.x * TILE_Z + threadIdx.x, y = blockIdx.y * TILE_Y + threadIdx.y;
+  const int x0 = blockIdx.z * kSpecPlanes, x1 = min(x0 + kSpecPlanes, g.nx);
+  if (z < g.pz && y < g.ny) {
+    for (int x = x0; x < x1; ++x) {
+      double div = 0.0;
+      if (interior(g, x, y, z)) {
+        const double tx = (ld(fx, x + 1, y, z) - ld(fx, x - 1, y, z)) * c2x;
+        const double ty = (ld(fy, x, y + 1, z) - ld(fy, x, y - 1, z)) * c2y;
+        const double tz = (ld(fz, x, y, z + 1) - ld(fz, x, y, z - 1)) * c2z;
+        div = (tx + ty) + tz;
+        mx = fmax(mx, fabs(div));
+      }
+      rhs[(long long)x * g.sxy + (long long)y * g.pz + z] = -div;
+    }
   }
-  // block max, then one atomic per block on the bit pattern (non-negative doubles)
-  __shared__ double red[32];
-  mx = warp_max(mx);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double v = threadIdx.x < (blockDim.x + 31) / 32 ? red[threadIdx.x] : 0.0;
-    v = warp_max(v);
-    if (threadIdx.x == 0)
-      atomicMax((unsigned long long*)maxdiv, (unsigned long long)__double_as_longlong(v));
-  }
+  // block max, then one atomic per block that raises it, on the bit pattern
+  // (non-negative doubles)
+  mx = block_max(mx, red);
+  if (flat_tid() == 0 && mx > *(volatile double*)maxdiv)
+    atomicMax((unsigned long long*)maxdiv, (unsigned long long)__double_as_longlong(mx));
 }
 
+// out = mask f - grad_c phi on interior cells (phi null: mask f), 0 elsewhere
 template <typename T>
-__global__ void finish_spectral(const T* __restrict__ fx, const T* __restrict__ fy,
-                                const T* __restrict__ fz, InStride s, Geom g, double c2x,
-                                double c2y, double c2z, const double* __restrict__ phi,
-                                double* __restrict__ out) {
-  const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int z = 1 + (int)(q % (g.nz - 2));
-    const long long r = q / (g.nz - 2);
-    const int y = 1 + (int)(r % (g.ny - 2));
-    const int x = 1 + (int)(r / (g.ny - 2));
+__global__ void __launch_bounds__(TILE_THREADS)
+    finish_spectral(const T* __restrict__ fx, const T* __restrict__ fy, const T* __restrict__ fz,
+                    InStride s, Geom g, double c2x, double c2y, double c2z,
+                    const double* __restrict__ phi, double* __restrict__ out) {
+  const int z = blockIdx.x * TILE_Z + threadIdx.x, y = blockIdx.y * TILE_Y + threadIdx.y;
+  const int x0 = blockIdx.z * kSpecPlanes, x1 = min(x0 + kSpecPlanes, g.nx);
+  if (z >= g.pz || y >= g.ny) return;
+  for (int x = x0; x < x1; ++x) {
     const long long i = (long long)x * g.sxy + (long long)y * g.pz + z;
-    const long long f = (long long)x * s.sx + (long long)y * s.sy + (long long)z * s.sz;
-    const double gx = (phi[i + g.sxy] - phi[i - g.sxy]) * c2x;
-    const double gy = (phi[i + g.pz] - phi[i - g.pz]) * c2y;
-    const double gz = (phi[i + 1] - phi[i - 1]) * c2z;
-    out[i] = (fx ? (double)fx[f] : 0.0) - gx;
-    out[i + g.ncell] = (fy ? (double)fy[f] : 0.0) - gy;
-    out[i + 2 * g.ncell] = (fz ? (double)fz[f] : 0.0) - gz;
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+    if (interior(g, x, y, z)) {
+      const long long f = (long long)x * s.sx + (long long)y * s.sy + (long long)z * s.sz;
+      double gx = 0.0, gy = 0.0, gz = 0.0;
+      if (phi) {
+        gx = (phi[i + g.sxy] - phi[i - g.sxy]) * c2x;
+        gy = (phi[i + g.pz] - phi[i - g.pz]) * c2y;
+        gz = (phi[i + 1] - phi[i - 1]) * c2z;
+      }
+      ox = (fx ? (double)fx[f] : 0.0) - gx;
+      oy = (fy ? (double)fy[f] : 0.0) - gy;
+      oz = (fz ? (double)fz[f] : 0.0) - gz;
+    }
+    out[i] = ox;
+    out[i + g.ncell] = oy;
+    out[i + 2 * g.ncell] = oz;
   }
 }
 
@@ -311,69 +503,74 @@ int spectral_one(const void* fx, const void* fy, const void* fz, InStride fs, co
   char* p = ws + 3 * vec;
   const int ns[3] = {g.nx, g.ny, g.nz};
   const double hs[3] = {dX, dY, dZ};
-  double* Q[3];
-  double* L[3];
-  cudaError_t e = cudaSuccess;
+  const bool has_interior = g.nx > 2 && g.ny > 2 && g.nz > 2;
+  if (!has_interior) {
+    if (cudaError_t e = cudaMemsetAsync(out, 0, (size_t)g.ncell * 3 * sizeof(double), s))
+      return cuda_status(e, "spectral setup");
+    if (stats) *stats = sw_cg_stats{0, SW_CG_EARLY_EXIT, 0.0, 0.0};
+    return SW_OK;
+  }
+  AxisBasis ax[3];
   for (int a = 0; a < 3; ++a) {
-    const int m = ns[a] > 2 ? ns[a] - 2 : 1;
-    Q[a] = (double*)p;
+    const int m = ns[a] - 2;
+    // the four chain matrices take at most m^2 + 1 values; m^2 + 1 > m^2 only
+    // for odd m, whose m^2 values leave room below the 256-byte boundary
+    double* q = (double*)p;
+    for (int par = 0; par < 2; ++par) ax[a].K[par] = chain_len(ns[a], par);
+    for (int dir = 0; dir < 2; ++dir)
+      for (int par = 0; par < 2; ++par) {
+        ax[a].W[dir][par] = q;
+        q += (size_t)ax[a].K[par] * ax[a].K[par];
+      }
     p += align_up((size_t)m * m * sizeof(double), 256);
-    L[a] = (double*)p;
+    ax[a].lam = (double*)p;
     p += align_up((size_t)m * sizeof(double), 256);
-    if (ns[a] > 2) {
-      const long long cnt = (long long)m * m;
-      axis_basis_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(ns[a], hs[a], Q[a], L[a]);
-      count_launches(1);
-      SW_CHECK_LAUNCH("spectral basis");
-    }
+    const long long cnt =
+        (long long)ax[a].K[0] * ax[a].K[0] + (long long)ax[a].K[1] * ax[a].K[1];
+    axis_basis_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>(ns[a], hs[a], ax[a]);
+    count_launches(1);
+    SW_CHECK_LAUNCH("spectral basis");
   }
   double* d_max = (double*)p;
-  if (e == cudaSuccess) e = cudaMemsetAsync(ws, 0, 3 * vec, s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_max, 0, sizeof(double), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, (size_t)g.ncell * 3 * sizeof(double), s);
+  cudaError_t e = cudaMemsetAsync(d_max, 0, sizeof(double), s);
   if (e != cudaSuccess) return cuda_status(e, "spectral setup");
   double maxdiv = 0.0;
-  const bool has_interior = g.nx > 2 && g.ny > 2 && g.nz > 2;
   const double c2x = 1.0 / (2.0 * dX), c2y = 1.0 / (2.0 * dY), c2z = 1.0 / (2.0 * dZ);
-  if (has_interior) {
-    const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-    const int grid = grid_blocks(n, 256, 148 * 16);
-    prep_rhs<T><<<grid, 256, 0, s>>>((const T*)fx, (const T*)fy, (const T*)fz, fs, g, c2x, c2y,
-                                     c2z, v0, d_max);
-    count_launches(1);
-    SW_CHECK_LAUNCH("spectral prep");
-    e = cudaMemcpyAsync(&maxdiv, d_max, sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_status(e, "spectral readback");
-  }
-  const bool solve = has_interior && !(maxdiv < 1e-12);
+  const dim3 blk(TILE_Z, TILE_Y);
+  prep_rhs<T><<<spec_grid(g), blk, 0, s>>>((const T*)fx, (const T*)fy, (const T*)fz, fs, g, c2x,
+                                           c2y, c2z, v0, d_max);
+  count_launches(1);
+  SW_CHECK_LAUNCH("spectral prep");
+  e = cudaMemcpyAsync(&maxdiv, d_max, sizeof(double), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_status(e, "spectral readback");
+  const bool solve = !(maxdiv < 1e-12);
   if (solve) {
-    // v0 -> v1 (x) -> v2 (y) -> v1 (z), scale, v1 -> v2 (z) -> v1 (y) -> v2 (x)
-    int rc = axis_transform(g, 0, Q[0], true, v0, v1, s);
-    if (rc == SW_OK) rc = axis_transform(g, 1, Q[1], true, v1, v2, s);
-    if (rc == SW_OK) rc = axis_transform(g, 2, Q[2], true, v2, v1, s);
-    if (rc != SW_OK) return rc;
+    // v0 -x-> v1 -y-> v2 -z-> v1 (scaled) -z-> v2 -y-> v1 -x-> v0.  Shell cells
+    // stay zero throughout without being cleared: axis x writes whole planes
+    // (from v0's zero shell), axis y whole rows, axis z the interior of lines
+    // whose ends axis x or y wrote; v0 keeps the shell planes of the rhs.
     double lmax = 0.0;
     for (int a = 0; a < 3; ++a) lmax += 4.0 / (hs[a] * hs[a]);
-    const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-    spectral_scale<<<grid_blocks(n, 256, 148 * 16), 256, 0, s>>>(v1, g, L[0], L[1], L[2],
-                                                                 1e-13 * lmax);
-    count_launches(1);
-    SW_CHECK_LAUNCH("spectral scale");
-    rc = axis_transform(g, 2, Q[2], false, v1, v2, s);
-    if (rc == SW_OK) rc = axis_transform(g, 1, Q[1], false, v2, v1, s);
-    if (rc == SW_OK) rc = cudaMemsetAsync(v2, 0, vec, s) == cudaSuccess ? SW_OK : SW_ECUDA;
-    if (rc == SW_OK) rc = axis_transform(g, 0, Q[0], false, v1, v2, s);
-    if (rc != SW_OK) return rc;
+    const double fl = 1e-13 * lmax;
+    struct {
+      int axis;
+      bool inverse, scale;
+      const double* src;
+      double* dst;
+    } const steps[6] = {{0, false, false, v0, v1}, {1, false, false, v1, v2},
+                        {2, false, true, v2, v1},  {2, true, false, v1, v2},
+                        {1, true, false, v2, v1},  {0, true, false, v1, v0}};
+    for (const auto& t : steps) {
+      const int rc = axis_transform(g, t.axis, ax[t.axis], t.inverse, t.src, t.dst, t.scale,
+                                    ax[0].lam, ax[1].lam, fl, s);
+      if (rc != SW_OK) return rc;
+    }
   }
-  if (has_interior) {
-    const long long n = (long long)(g.nx - 2) * (g.ny - 2) * (g.nz - 2);
-    finish_spectral<T><<<grid_blocks(n, 256, 148 * 16), 256, 0, s>>>(
-        (const T*)fx, (const T*)fy, (const T*)fz, fs, g, c2x, c2y, c2z,
-        solve ? v2 : v1 /* zero field when no solve */, out);
-    count_launches(1);
-    SW_CHECK_LAUNCH("spectral finish");
-  }
+  finish_spectral<T><<<spec_grid(g), blk, 0, s>>>((const T*)fx, (const T*)fy, (const T*)fz, fs, g,
+                                                  c2x, c2y, c2z, solve ? v0 : nullptr, out);
+  count_launches(1);
+  SW_CHECK_LAUNCH("spectral finish");
   if (stats) {
     stats->iters = 0;
     stats->reason = solve ? SW_CG_CONVERGED : SW_CG_EARLY_EXIT;
