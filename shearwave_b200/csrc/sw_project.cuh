@@ -10,19 +10,17 @@ struct InStride {
   long long sx, sy, sz;
 };
 
-// Scalar state of one CG solve, advanced on the device by the last block of
-// each launch.
+// Scalar state of one CG solve, recorded on the device.
 struct CgState {
-  double rs;      // r.r of the current residual (rs_old)
+  double rs[2];   // r.r of the residual before iteration k in rs[k & 1]
   double rs0;     // max(r0.r0, eps64)
-  double alpha, beta;
   double rel;     // sqrt(rs_new / rs0) of the last update
   double maxdiv;  // max |div_c f| of the masked input
   double tol;
   int iters;      // completed x updates
   int reason;     // enum sw_cg_reason
-  int k;          // index of the next apply (selects the p buffer)
   int max_iters;
+  int brk;        // the last p.Ap ended the iteration (breakdown); -1: a wait ran out
   unsigned int ticket;
 };
 
@@ -47,11 +45,13 @@ inline CgGrid* cg_grid_of(CgState* st) { return (CgGrid*)((char*)st + 128); }
 //         reference's elastic_solve_static loop (solver.py:605-623).
 struct CgInst {
   Geom g;
-  TileSpace ts;
+  TileSpace ts;          // tiles of cg_prep and cg_finish
+  int ring_base;         // first tile of this instance in cg_ring
   double c2x, c2y, c2z;  // 1 / (2 h)
   double ihx2, ihy2, ihz2;  // 1 / h^2 (op 1)
-  double *x, *r, *p0, *p1, *ap;
-  double* muf;           // mu on interior cells, FP64 (op 1)
+  double *x, *r, *p0, *p1;
+  double* ap;            // holds the solve's CgRing (A p is recomputed, not stored)
+  double* muf;           // mu on interior cells, FP64 (op 1; null: mu_s)
   double mu_s;           // scalar mu when no field is given (op 1)
   double2* partials;     // per tile: (sum, max)
   CgState* st;

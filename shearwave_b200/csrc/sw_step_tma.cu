@@ -57,18 +57,22 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const uint64_t dims[4],
-                   const uint64_t strides_bytes[3], const uint32_t box[4]) {
+static int encode_tmap(int rank, CUtensorMap* map, CUtensorMapDataType dt, void* base,
+                       const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return SW_ECUDA;
   }
-  cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]};
-  cuuint64_t s[3] = {strides_bytes[0], strides_bytes[1], strides_bytes[2]};
-  cuuint32_t b[4] = {box[0], box[1], box[2], box[3]};
-  cuuint32_t e[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, dt, 4, base, d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  cuuint64_t d[4], s[4];
+  cuuint32_t b[4], e[4];
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    e[i] = 1;
+    if (i + 1 < rank) s[i] = strides_bytes[i];
+  }
+  CUresult r = fn(map, dt, (cuuint32_t)rank, base, d, s, b, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
@@ -76,6 +80,16 @@ int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const u
     return SW_ECUDA;
   }
   return SW_OK;
+}
+
+int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const uint64_t dims[4],
+                   const uint64_t strides_bytes[3], const uint32_t box[4]) {
+  return encode_tmap(4, map, dt, base, dims, strides_bytes, box);
+}
+
+int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const uint64_t dims[3],
+                   const uint64_t strides_bytes[2], const uint32_t box[3]) {
+  return encode_tmap(3, map, dt, base, dims, strides_bytes, box);
 }
 
 // ---------------------------------------------------------------------------

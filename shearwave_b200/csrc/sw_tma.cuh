@@ -73,6 +73,16 @@ __device__ inline void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* 
       : "memory");
 }
 
+// 3-D form of tma_load_4d.
+__device__ inline void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0,
+                                   int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(bar))
+      : "memory");
+}
+
 __device__ inline void prefetch_tmap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -279,5 +289,8 @@ __device__ inline bool consumer_sync_or(bool fail, int nthreads) {
 // bytes for dims 1..3).  Returns a CUDA driver status.
 int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const uint64_t dims[4],
                    const uint64_t strides_bytes[3], const uint32_t box[4]);
+// The same for a 3-D map.
+int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, void* base, const uint64_t dims[3],
+                   const uint64_t strides_bytes[2], const uint32_t box[3]);
 
 }  // namespace sw
