@@ -165,12 +165,15 @@ __global__ void __launch_bounds__(TILE_THREADS) cg_prep(const CgInst* __restrict
 // from shared memory.  The update phase walks x the other way, starting with
 // the planes the apply phase left in L2.  Two blocks per SM.  Measured against
 // a walk with every stencil point from global memory: an iteration at 192^3
-// takes 90 instead of 160 us (DRAM bytes alone 69), the 442 of a static solve
-// at 121 x 121 x 141 16.1 instead of 31.6 ms.
-// Stages: planes x, x +- 1, x +- 2 held, the rest in flight.  A stage holds
-// the boxes of p and r in the apply phase; in the update phase the same room
-// holds a ring of p boxes and one of point-wise planes.
-constexpr int CR_NA = 8, CR_NB = CR_NA - 2;
+// takes 86 instead of 160 us (DRAM bytes alone 69; 6 TB/s while the tiles
+// walk, the rest is the phases' ends), the 442 of a static solve at 121 x 121
+// x 141, whose vectors fit L2, 13.6 instead of 31.6 ms.
+// The walk goes by units of two planes (one barrier, and two independent
+// stencils for a thread to overlap).  Stages: the unit in work and the one
+// ahead held, two in flight.  A stage holds the boxes of p and r in the apply
+// phase; in the update phase the same room holds a ring of p boxes and one of
+// point-wise planes.
+constexpr int CR_NA = 4, CR_NB = CR_NA - 1;
 template <int LZ>
 struct CrShape {
   static constexpr int LY = 512 / LZ;  // tile LZ x LY, a warp 64 / LZ rows of LZ / 2 pairs
@@ -180,8 +183,8 @@ struct CrShape {
 constexpr int CR_BOX = CrShape<64>::BOX > CrShape<32>::BOX ? CrShape<64>::BOX : CrShape<32>::BOX;
 constexpr int CR_PT = 512;  // cells of a point box
 constexpr int CR_WARPS = 8, CR_THREADS = 32 * (CR_WARPS + 1);
-constexpr size_t CR_RINGS = sizeof(double) * (2 * CR_NA * CR_BOX);
-static_assert(sizeof(double) * (CR_NA * CR_BOX + 2 * CR_NB * CR_PT) <= CR_RINGS,
+constexpr size_t CR_RINGS = sizeof(double) * (4 * CR_NA * CR_BOX);
+static_assert(sizeof(double) * (2 * CR_NA * CR_BOX + 4 * CR_NB * CR_PT) <= CR_RINGS,
               "the update phase's rings take the apply phase's room");
 constexpr size_t CR_SMEM = 128 + kRingOffset + CR_RINGS;
 static_assert(2 * (CR_SMEM + 1024) <= 233472, "two blocks must fit one SM");
@@ -206,306 +209,374 @@ __device__ __forceinline__ double2 fma2(double a, double2 b, double2 c) {
 
 struct CgHeader {
   uint64_t full[CR_NA], empty[CR_NA];
+  uint64_t sync;  // consumer_sync
 };
 static_assert(sizeof(CgHeader) <= kAbortFlagOffset, "header overlaps the abort flag");
 
 // Shared-memory view and ring position of one thread's role in a block.
 struct CgPipe {
-  double* rings;  // apply: [stage][p box, r box]; update: [stage][p box], [stage][x box, r box]
+  // apply: [stage][p box pair, r box pair]; update: [stage][p box pair], then
+  // [stage][x pair, r pair]
+  double* rings;
   CgHeader* hd;
   volatile int* abort_flag;
   RingPos<CR_NA> a;
   int b = 0;
+  uint32_t sync_ph = 0;
   template <bool UPDATE>
   __device__ double* stage(int st) const {
-    return rings + st * (UPDATE ? CR_BOX : 2 * CR_BOX);
+    return rings + st * (UPDATE ? 2 * CR_BOX : 4 * CR_BOX);
   }
-  __device__ double* points() const { return rings + CR_NA * CR_BOX + b * 2 * CR_PT; }
+  __device__ double* points() const { return rings + CR_NA * 2 * CR_BOX + b * 4 * CR_PT; }
   __device__ void next_points() { b = b + 1 == CR_NB ? 0 : b + 1; }
 };
 
-// Producer: the planes of one tile in walk order, n + 4 of ring A (two halo
-// planes either side); in the update phase the point-wise planes of the n
-// planes, each on the barrier of the plane two ahead.  (Their ring needs no
-// barrier for its reuse: a free stage means that the plane CR_NA - 2 = CR_NB
-// before the point-wise one being loaded is done.)
+// What a block keeps of the instance it works on (shared memory).  The scalars
+// follow the iteration as the owner's record does (every block computes the
+// same), so a block that stays with one instance reads the record once: with
+// every warp of every block reading it in each phase, its few L2 lines were
+// the longest part of a phase's start (6300 cycles of a 37000-cycle phase at
+// 121 x 121 x 141; now 4100 that overlap the first loads).
+struct CgCache {
+  CgInst in;
+  TileSpace tr;
+  int lz;
+  int inst;     // its table index
+  int run;      // whether this phase works on it, and its beta or alpha
+  double scal;
+  double rs, rs0, tol;  // rs: r.r of the residual before the current iteration
+  int reason, brk, max_iters;
+};
+
+// The producer's tile, looked up when it changes.
+struct CgTile {
+  const CgRing* rg;
+  const CgState* st;
+  TileCoord tc;
+  int t, lz;
+};
+
+// Producer: the units of one tile in walk order: one behind, U = ceil(n / 2),
+// one ahead (unit u holds planes 2u and 2u + 1 of the walk); in the update
+// phase the point-wise planes of a unit, on the barrier of the unit ahead.
+// (Their ring needs no barrier for its reuse: a free stage means that the unit
+// CR_NA - 1 = CR_NB before the point-wise one being loaded is done.)  Of a
+// last unit with one plane of the tile the other plane is loaded too and never
+// used.  The tile's number goes with its first unit.
 template <bool UPDATE>
 __device__ __forceinline__ bool ring_load(const CgRing* __restrict__ rg, const TileCoord& tc,
-                                          int k, CgPipe& q, AbortLog* lg) {
+                                          int t, int lz, int k, CgPipe& q, AbortLog* lg,
+                                          volatile int* slots) {
   const CUtensorMap* pm = UPDATE ? &rg->ph[k & 1] : &rg->ph[(k & 1) ^ 1];
-  const uint32_t box = 8u * (rg->lz == 32 ? CrShape<32>::BOX : CrShape<64>::BOX);
-  const int n = tc.x1 - tc.x0;
-  for (int j = -2; j < n + 2; ++j) {
-    const int x = UPDATE ? tc.x1 - 1 - j : tc.x0 + j;
-    if (!ws_wait(&q.hd->empty[q.a.s], q.a.ph ^ 1u, q.abort_flag)) return false;
-    double* A = q.stage<UPDATE>(q.a.s);
-    uint64_t* full = &q.hd->full[q.a.s];
-    const bool points = UPDATE && j >= 2;
+  const uint32_t box = 16u * (lz == 32 ? CrShape<32>::BOX : CrShape<64>::BOX);
+  const int U = (tc.x1 - tc.x0 + 1) / 2;
+  for (int u = -1; u <= U; ++u) {
+    // lower plane of the pair
+    const int x = UPDATE ? tc.x1 - 2 - 2 * u : tc.x0 + 2 * u;
+    const int st = q.a.s;
+    if (!ws_wait(&q.hd->empty[st], q.a.ph ^ 1u, q.abort_flag)) return false;
+    double* A = q.stage<UPDATE>(st);
+    uint64_t* full = &q.hd->full[st];
+    const bool points = UPDATE && u >= 1;
+    if (u == -1) slots[st] = t;
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(full, UPDATE ? box + (points ? 16u * CR_PT : 0u) : 2u * box);
+    mbar_arrive_expect_tx(full, UPDATE ? box + (points ? 32u * CR_PT : 0u) : 2u * box);
     tma_load_3d(A, pm, full, tc.z0 - 2, tc.y0 - 2, x);
-    if (!UPDATE) tma_load_3d(A + CR_BOX, &rg->rh, full, tc.z0 - 2, tc.y0 - 2, x);
+    if (!UPDATE) tma_load_3d(A + 2 * CR_BOX, &rg->rh, full, tc.z0 - 2, tc.y0 - 2, x);
     if (points) {
       double* B = q.points();
       tma_load_3d(B, &rg->xp, full, tc.z0, tc.y0, x + 2);
-      tma_load_3d(B + CR_PT, &rg->rp, full, tc.z0, tc.y0, x + 2);
+      tma_load_3d(B + 2 * CR_PT, &rg->rp, full, tc.z0, tc.y0, x + 2);
       q.next_points();
     }
-    arm_record(lg->armedA, lg->parA, q.a.s, q.a.ph);
+    arm_record(lg->armedA, lg->parA, st, q.a.ph);
     q.a.next();
   }
   return true;
 }
 
-// Consumer: one tile for one warp.  `scal` is beta (apply) or alpha (update);
-// acc receives the thread's partial of the phase's sum.
+// Consumer: one tile for one warp; the first unit's barrier has been waited
+// for.  `scal` is beta (apply) or alpha (update); acc receives the thread's
+// partial of the phase's sum.
 template <int LZ, int OP, bool UPDATE>
 __device__ __forceinline__ bool ring_tile(const CgInst& in, const TileCoord& tc, int k,
                                           double scal, CgPipe& q, int w, int lane, double* acc) {
   using S = CrShape<LZ>;
   constexpr int W = S::W;
-  const Geom g = in.g;
+  // the walk's first and second plane of a unit in its boxes (halo, point)
+  constexpr int I0 = UPDATE ? S::BOX : 0, I1 = UPDATE ? 0 : S::BOX;
+  constexpr int B0 = UPDATE ? CR_PT : 0, B1 = UPDATE ? 0 : CR_PT;
+  const int nx = in.g.nx, ny = in.g.ny, nz = in.g.nz;
+  const long long sxy = in.g.sxy;
   const int row = LZ == 64 ? w : 2 * w + (lane >> 4), zl = LZ == 64 ? 2 * lane : 2 * (lane & 15);
   const int y = tc.y0 + row, z = tc.z0 + zl;
-  const bool yin = y >= 1 && y <= g.ny - 2;
-  const bool aa = yin && z >= 1 && z <= g.nz - 2, ab = yin && z + 1 <= g.nz - 2;
+  const bool yin = y >= 1 && y <= ny - 2;
+  const bool aa = yin && z >= 1 && z <= nz - 2, ab = yin && z + 1 <= nz - 2;
   const int o = (row + 2) * W + 2 + zl, ob = row * LZ + zl;
   const double cx = in.c2x, cy = in.c2y, cz = in.c2z;
   // a gradient whose centre lies on the shell is dropped: zero coefficients
-  const double cyp = y + 1 <= g.ny - 2 ? cy : 0.0, cym = y - 1 >= 1 ? cy : 0.0;
-  const double czpa = z + 1 <= g.nz - 2 ? cz : 0.0, czma = z - 1 >= 1 ? cz : 0.0;
-  const double czpb = z + 2 <= g.nz - 2 ? cz : 0.0, czmb = z >= 1 ? cz : 0.0;
-  const double hx = in.ihx2, hy = in.ihy2, hz = in.ihz2, mu_s = in.mu_s;  // op 1
-  const double* __restrict__ muf = in.muf;
-  double* __restrict__ pn = (k & 1) ? in.p1 : in.p0;
-  double* __restrict__ X = in.x;
+  const double cyp = y + 1 <= ny - 2 ? cy : 0.0, cym = y - 1 >= 1 ? cy : 0.0;
+  const double czpa = z + 1 <= nz - 2 ? cz : 0.0, czma = z - 1 >= 1 ? cz : 0.0;
+  const double czpb = z + 2 <= nz - 2 ? cz : 0.0, czmb = z >= 1 ? cz : 0.0;
+  double* __restrict__ X = UPDATE ? in.x : ((k & 1) ? in.p1 : in.p0);
   double* __restrict__ R = in.r;
   auto value = [&](const double* A, int i) -> double2 {  // p at a pair of a stage
     const double2 p = ld2(A + i);
-    return UPDATE ? p : fma2(scal, p, ld2(A + CR_BOX + i));
-  };
-  auto next = [&](double2* v) -> bool {  // the own pair of the next plane
-    const int st = q.a.s;
-    if (!ws_wait(&q.hd->full[st], q.a.ph, q.abort_flag)) return false;
-    q.a.next();
-    *v = value(q.stage<UPDATE>(st), o);
-    return true;
+    return UPDATE ? p : fma2(scal, p, ld2(A + 2 * CR_BOX + i));
   };
   auto release = [&](int st) {
     __syncwarp();
     if (lane == 0) mbar_arrive(&q.hd->empty[st]);
   };
   const int n = tc.x1 - tc.x0, xs = UPDATE ? tc.x1 - 1 : tc.x0;  // first plane of the walk
-  int s0 = q.a.s;
-  auto advance = [&]() { s0 = s0 + 1 == CR_NA ? 0 : s0 + 1; };
-  double2 b2, b1, pc, f1;
-  if (!next(&b2)) return false;  // the two planes behind the walk: own pair only
-  release(s0);
-  advance();
-  if (!next(&b1)) return false;
-  release(s0);
-  advance();
-  if (!next(&pc) || !next(&f1)) return false;
-  long long i = (long long)xs * g.sxy + (long long)y * g.pz + z;
-  double sum = 0.0;
-  // new x and r (update) or p (apply) at the plane, its sum, and its release
-  auto finish = [&](double2 c, double2 ap) {
-    release(s0);
-    advance();
-    if (UPDATE) {
-      const double* B = q.points();
-      q.next_points();
-      const double2 xn = fma2(scal, c, ld2(B + ob));
-      const double2 rn = fma2(-scal, ap, ld2(B + CR_PT + ob));
-      if (aa && ab) {
-        *reinterpret_cast<double2*>(X + i) = xn;
-        *reinterpret_cast<double2*>(R + i) = rn;
-      } else if (aa) {
-        X[i] = xn.x;
-        R[i] = rn.x;
-      } else if (ab) {
-        X[i + 1] = xn.y;
-        R[i + 1] = rn.y;
-      }
-      if (aa) sum = fma(rn.x, rn.x, sum);
-      if (ab) sum = fma(rn.y, rn.y, sum);
-      i -= g.sxy;
-    } else {
-      if (aa && ab) *reinterpret_cast<double2*>(pn + i) = c;
-      else if (aa) pn[i] = c.x;
-      else if (ab) pn[i + 1] = c.y;
-      if (aa) sum = fma(c.x, ap.x, sum);
-      if (ab) sum = fma(c.y, ap.y, sum);
-      i += g.sxy;
-    }
-  };
-  if (OP == 0) {
-    // gradients towards the planes behind: centre one plane behind xs, and xs
-    // itself (interior) for the second plane
-    const double c0 = (UPDATE ? xs + 1 <= g.nx - 2 : xs - 1 >= 1) ? cx : 0.0;
-    auto grad = [](double2 on, double2 back, double c) {
-      return make_double2((on.x - back.x) * c, (on.y - back.y) * c);
-    };
-    double2 ga = UPDATE ? grad(b2, pc, c0) : grad(pc, b2, c0);
-    double2 gb = UPDATE ? grad(b1, f1, cx) : grad(f1, b1, cx);
-    auto plane = [&](int j, double2& c, double2& gx) -> bool {
-      const double* A = q.stage<UPDATE>(s0);
-      double2 f2;
-      if (!next(&f2)) return false;
-      const double2 N = value(A, o + 2 * W), Sv = value(A, o - 2 * W);
-      const double2 L = value(A, o - 2), Rv = value(A, o + 2);
-      const double ca = (UPDATE ? xs - j - 1 >= 1 : xs + j + 1 <= g.nx - 2) ? cx : 0.0;
-      const double2 go = UPDATE ? grad(c, f2, ca) : grad(f2, c, ca);  // ahead of the walk
-      double2 ap;
-      {
-        const double tx = (UPDATE ? gx.x - go.x : go.x - gx.x) * cx;
-        const double ty = ((N.x - c.x) * cyp - (c.x - Sv.x) * cym) * cy;
-        const double tz = ((Rv.x - c.x) * czpa - (c.x - L.x) * czma) * cz;
-        ap.x = -((tx + ty) + tz);
-      }
-      {
-        const double tx = (UPDATE ? gx.y - go.y : go.y - gx.y) * cx;
-        const double ty = ((N.y - c.y) * cyp - (c.y - Sv.y) * cym) * cy;
-        const double tz = ((Rv.y - c.y) * czpb - (c.y - L.y) * czmb) * cz;
-        ap.y = -((tx + ty) + tz);
-      }
-      finish(c, ap);
-      c = f2;
-      gx = go;
-      return true;
-    };
-    for (int j = 0; j < n; j += 2) {
-      if (!plane(j, pc, ga)) return false;
-      if (j + 1 < n && !plane(j + 1, f1, gb)) return false;
-    }
-  } else {
-    for (int j = 0; j < n; ++j) {
-      double2 mu = make_double2(mu_s, mu_s);
-      if (muf != nullptr && (aa || ab)) mu = ld2(muf + i);
-      const double* A = q.stage<UPDATE>(s0);
-      double2 f2;
-      if (!next(&f2)) return false;
-      const double2 N = value(A, o + W), Sv = value(A, o - W);
-      const double2 L = value(A, o - 2), Rv = value(A, o + 2);
-      const double2 hi = UPDATE ? b1 : f1, lo = UPDATE ? f1 : b1;
-      double2 ap;
-      ap.x = -mu.x * (((hi.x - 2.0 * pc.x) + lo.x) * hx + ((N.x - 2.0 * pc.x) + Sv.x) * hy +
-                      ((pc.y - 2.0 * pc.x) + L.y) * hz);
-      ap.y = -mu.y * (((hi.y - 2.0 * pc.y) + lo.y) * hx + ((N.y - 2.0 * pc.y) + Sv.y) * hy +
-                      ((Rv.x - 2.0 * pc.y) + pc.x) * hz);
-      finish(pc, ap);
-      b1 = pc;
-      pc = f1;
-      f1 = f2;
-    }
+  const long long step = UPDATE ? -sxy : sxy;
+  double2 g0, g1;  // the two planes behind the walk, then gradients towards them
+  {
+    const double* A = q.stage<UPDATE>(q.a.s);
+    g0 = value(A, I0 + o);
+    g1 = value(A, I1 + o);
+    release(q.a.s);
+    q.a.next();
   }
-  release(s0);  // the two planes ahead of the walk
-  advance();
-  release(s0);
+  int s0 = q.a.s;
+  if (!ws_wait(&q.hd->full[s0], q.a.ph, q.abort_flag)) return false;
+  q.a.next();
+  double2 c0, c1;  // the unit's own pairs
+  {
+    const double* A = q.stage<UPDATE>(s0);
+    c0 = value(A, I0 + o);
+    c1 = value(A, I1 + o);
+  }
+  auto grad = [](double2 on, double2 back, double c) {
+    return make_double2((on.x - back.x) * c, (on.y - back.y) * c);
+  };
+  const double2 behind = g1;  // op 1: the plane behind the walk
+  if (OP == 0) {
+    // centres: one plane behind xs, and xs itself (interior)
+    const double cb = (UPDATE ? xs + 1 <= nx - 2 : xs - 1 >= 1) ? cx : 0.0;
+    g0 = UPDATE ? grad(g0, c0, cb) : grad(c0, g0, cb);
+    g1 = UPDATE ? grad(g1, c1, cx) : grad(c1, g1, cx);
+  }
+  double2 bk = behind;
+  long long i = (long long)xs * sxy + (long long)y * in.g.pz + z;
+  double sum = 0.0;
+  // A p at one plane of op 0: gx the x gradient behind, go the one ahead
+  auto stencil0 = [&](const double* A, double2 c, double2 gx, double2 go) -> double2 {
+    const double2 N = value(A, o + 2 * W), Sv = value(A, o - 2 * W);
+    const double2 L = value(A, o - 2), Rv = value(A, o + 2);
+    double2 ap;
+    {
+      const double tx = (UPDATE ? gx.x - go.x : go.x - gx.x) * cx;
+      const double ty = ((N.x - c.x) * cyp - (c.x - Sv.x) * cym) * cy;
+      const double tz = ((Rv.x - c.x) * czpa - (c.x - L.x) * czma) * cz;
+      ap.x = -((tx + ty) + tz);
+    }
+    {
+      const double tx = (UPDATE ? gx.y - go.y : go.y - gx.y) * cx;
+      const double ty = ((N.y - c.y) * cyp - (c.y - Sv.y) * cym) * cy;
+      const double tz = ((Rv.y - c.y) * czpb - (c.y - L.y) * czmb) * cz;
+      ap.y = -((tx + ty) + tz);
+    }
+    return ap;
+  };
+  // A p at one plane of op 1: xa, xb its x neighbours (either order)
+  auto stencil1 = [&](const double* A, double2 c, double2 xa, double2 xb, long long at) -> double2 {
+    const double hx = in.ihx2, hy = in.ihy2, hz = in.ihz2;
+    double2 mu = make_double2(in.mu_s, in.mu_s);
+    if (in.muf != nullptr && (aa || ab)) mu = ld2(in.muf + at);
+    const double2 N = value(A, o + W), Sv = value(A, o - W);
+    const double2 L = value(A, o - 2), Rv = value(A, o + 2);
+    const double2 hi = UPDATE ? xa : xb, lo = UPDATE ? xb : xa;
+    double2 ap;
+    ap.x = -mu.x * (((hi.x - 2.0 * c.x) + lo.x) * hx + ((N.x - 2.0 * c.x) + Sv.x) * hy +
+                    ((c.y - 2.0 * c.x) + L.y) * hz);
+    ap.y = -mu.y * (((hi.y - 2.0 * c.y) + lo.y) * hx + ((N.y - 2.0 * c.y) + Sv.y) * hy +
+                    ((Rv.x - 2.0 * c.y) + c.x) * hz);
+    return ap;
+  };
+  // new x and r (update) or p (apply) of one plane, and its sum
+  auto finish = [&](double2 c, double2 ap, const double* B, long long at, bool wa, bool wb) {
+    double2 v, rn;
+    if (UPDATE) {
+      v = fma2(scal, c, ld2(B + ob));
+      rn = fma2(-scal, ap, ld2(B + 2 * CR_PT + ob));
+    } else {
+      v = c;
+    }
+    if (wa && wb) {
+      *reinterpret_cast<double2*>(X + at) = v;
+      if (UPDATE) *reinterpret_cast<double2*>(R + at) = rn;
+    } else if (wa) {
+      X[at] = v.x;
+      if (UPDATE) R[at] = rn.x;
+    } else if (wb) {
+      X[at + 1] = v.y;
+      if (UPDATE) R[at + 1] = rn.y;
+    }
+    if (wa) sum = UPDATE ? fma(rn.x, rn.x, sum) : fma(c.x, ap.x, sum);
+    if (wb) sum = UPDATE ? fma(rn.y, rn.y, sum) : fma(c.y, ap.y, sum);
+  };
+  for (int j = 0; j < n; j += 2, i += 2 * step) {
+    const int s1 = q.a.s;  // the unit ahead
+    if (!ws_wait(&q.hd->full[s1], q.a.ph, q.abort_flag)) return false;
+    q.a.next();
+    const bool two = j + 1 < n;
+    const double* A = q.stage<UPDATE>(s0);
+    const double* An = q.stage<UPDATE>(s1);
+    const double2 f0 = value(An, I0 + o), f1 = value(An, I1 + o);
+    double2 ap0, ap1;
+    if (OP == 0) {
+      const double ca0 = (UPDATE ? xs - j - 1 >= 1 : xs + j + 1 <= nx - 2) ? cx : 0.0;
+      const double ca1 = (UPDATE ? xs - j - 2 >= 1 : xs + j + 2 <= nx - 2) ? cx : 0.0;
+      const double2 go0 = UPDATE ? grad(c0, f0, ca0) : grad(f0, c0, ca0);
+      const double2 go1 = UPDATE ? grad(c1, f1, ca1) : grad(f1, c1, ca1);
+      ap0 = stencil0(A + I0, c0, g0, go0);
+      ap1 = stencil0(A + I1, c1, g1, go1);
+      g0 = go0;
+      g1 = go1;
+    } else {
+      ap0 = stencil1(A + I0, c0, bk, c1, i);
+      ap1 = stencil1(A + I1, c1, c0, f0, two ? i + step : i);
+      bk = c1;
+    }
+    release(s0);
+    const double* B = q.points();
+    finish(c0, ap0, B + B0, i, aa, ab);
+    finish(c1, ap1, B + B1, i + step, aa && two, ab && two);
+    if (UPDATE) q.next_points();
+    c0 = f0;
+    c1 = f1;
+    s0 = s1;
+  }
+  release(s0);  // the unit ahead of the walk
   *acc = sum;
   return true;
 }
 
-// Grid-wide barrier (every block of the cooperative launch); bounded, and an
-// error raised by any block ends it.
-__device__ bool cg_grid_sync(CgGrid* b) {
-  __shared__ int ok_s;
+// Grid-wide barrier number n = 1, 2, ... (every block of the cooperative
+// launch): arrivals are counted in one word, the last one raises the other,
+// which the waiting blocks poll (on a line of its own, so the polls do not
+// hold up the arrivals).  Bounded; an error raised by any block, or a wait
+// that ran out in this one, ends it.
+__device__ __forceinline__ bool cg_grid_sync(CgGrid b, unsigned int n, volatile int* abort_flag,
+                                             int* ok_s) {
   asm volatile("fence.proxy.async;" ::: "memory");  // this phase's stores, next phase's TMA reads
-  __threadfence();
   __syncthreads();
+  if (*abort_flag) return false;  // the same in every thread: set before the barrier, if at all
   if (threadIdx.x == 0) {
     int ok = 1;
-    volatile unsigned int* gen = &b->gen;
-    const unsigned int g0 = *gen;
-    __threadfence();
-    if (atomicAdd(&b->count, 1u) + 1u == gridDim.x) {
-      atomicExch(&b->count, 0u);
-      __threadfence();
-      atomicAdd(&b->gen, 1u);
+    unsigned int v;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                 : "=r"(v)
+                 : "l"(b.count)
+                 : "memory");
+    if (v + 1u == n * gridDim.x) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(b.gen) : "memory");
     } else {
       const uint32_t t0 = (uint32_t)clock();
-      while (*gen == g0) {
-        if (*(volatile int*)&b->error) {
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(b.gen) : "memory");
+        if (v & kCgGridError) {
           ok = 0;
           break;
         }
+        if ((int)((v << 1) - (n << 1)) >= 0) break;
         if ((((uint32_t)clock() - t0) >> 10) > kCgWaitBudget) {
-          atomicExch(&b->error, 1);
+          atomicOr(b.gen, kCgGridError);
           ok = 0;
           break;
         }
       }
     }
-    __threadfence();
-    ok_s = ok;
+    *ok_s = ok;
   }
   __syncthreads();
   asm volatile("fence.proxy.async;" ::: "memory");
-  return ok_s != 0;
+  return *ok_s != 0;
 }
 
-// Start of a phase for one instance, in every block that has one of its tiles
-// (all threads): sums the other phase's partials and applies the stopping
-// rule; every block computes the same values.  Returns in `run` whether the
-// phase works on the instance and in `scal` its beta (apply) or alpha
-// (update).  The owner records the scalars: `reason` changes in apply phases
-// only and `brk` in update phases only, so nobody reads a word in the phase
-// that writes it except to reach the decision it holds.
-__device__ __forceinline__ void cg_phase_begin(const CgInst& in, bool update, int k, bool owner,
-                                               double* red, int* run_s, double* scal_s) {
+// Barrier of the consumer warps; bounded, false once a wait of the block has
+// run out.
+constexpr int CR_CTHREADS = 32 * CR_WARPS;
+__device__ __forceinline__ bool consumer_sync(CgPipe& q) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(&q.hd->sync);
+  const bool ok = ws_wait(&q.hd->sync, q.sync_ph, q.abort_flag);
+  q.sync_ph ^= 1u;
+  return ok;
+}
+
+// Per-tile partials of a phase: p.Ap (apply), r.r (update).
+__device__ __forceinline__ double* cg_partials(const CgInst& in, bool update) {
+  return reinterpret_cast<double*>(in.partials) + (update ? in.ts.count : 0);
+}
+
+// Start of a phase for the cached instance, in every block that has one of its
+// tiles (the consumer threads): sums the other phase's partials and applies
+// the stopping rule; every block computes the same values.  Sets cc->run
+// (whether the phase works on the instance) and cc->scal (its beta in apply
+// phases, alpha in update phases).  The owner records the scalars: `reason`
+// changes in apply phases only and `brk` in update phases only, so nobody
+// reads a word in the phase that writes it except to reach the decision it
+// holds.
+__device__ __forceinline__ bool cg_phase_begin(CgCache* cc, bool update, int k, bool owner,
+                                               double* red, CgPipe& q) {
+  const CgInst& in = cc->in;
   CgState* st = in.st;
   double v = 0.0;
   if (update || k > 0) {
-    const CgRing* rg = reinterpret_cast<const CgRing*>(in.ap);
-    const int n = rg->tr.count;
-    const double* pp = reinterpret_cast<const double*>(in.partials);
-    for (int i = threadIdx.x; i < n; i += CR_THREADS) v += __ldcg(pp + 2 * i + (update ? 0 : 1));
+    const double* pp = cg_partials(in, !update);
+    for (int i = threadIdx.x; i < cc->tr.count; i += CR_CTHREADS) v += __ldcg(pp + i);
   }
-  const int reason = __ldcg(&st->reason), brk = __ldcg(&st->brk);
-  const double rs = __ldcg(&st->rs[update ? (k & 1) : ((k - 1) & 1)]);
-  v = block_sum(v, red);
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  if (!consumer_sync(q)) return false;
   if (threadIdx.x == 0) {
-    int run = reason == SW_CG_RUNNING;
+    v = 0.0;
+#pragma unroll
+    for (int w = 0; w < CR_WARPS; ++w) v += red[w];
+    int run = cc->reason == SW_CG_RUNNING;
     double scal = 0.0;
     if (run && update) {
-      const double denom = v;
-      const bool stop = in.op == 1 ? denom <= 0.0 : (!isfinite(denom) || denom <= 0.0);
+      const bool stop = in.op == 1 ? v <= 0.0 : (!isfinite(v) || v <= 0.0);
       if (stop) {
+        cc->brk = 1;
         if (owner) st->brk = 1;
         run = 0;
       } else {
-        scal = rs / denom;
+        scal = cc->rs / v;
       }
     } else if (run) {
-      if (brk) {
-        if (owner) st->reason = SW_CG_BREAKDOWN;
-        run = 0;
+      int why = SW_CG_RUNNING;
+      if (cc->brk) {
+        why = SW_CG_BREAKDOWN;
       } else if (k > 0) {
         if (owner) st->iters = k;
         if (in.op == 0 && !isfinite(v)) {
-          if (owner) st->reason = SW_CG_NONFINITE;
-          run = 0;
+          why = SW_CG_NONFINITE;
         } else {
-          const double rel = sqrt(v / st->rs0);
+          const double rel = sqrt(v / cc->rs0);
+          scal = v / fmax(cc->rs, 2.220446049250313e-16);
           if (owner) st->rel = rel;
-          if (rel < st->tol) {
-            if (owner) st->reason = SW_CG_CONVERGED;
-            run = 0;
+          if (rel < cc->tol) {
+            why = SW_CG_CONVERGED;
           } else {
-            scal = v / fmax(rs, 2.220446049250313e-16);
             if (owner) st->rs[k & 1] = v;
-            if (k >= st->max_iters) {
-              if (owner) st->reason = SW_CG_MAXITERS;
-              run = 0;
-            }
+            cc->rs = v;
+            if (k >= cc->max_iters) why = SW_CG_MAXITERS;
           }
         }
       }
+      if (why != SW_CG_RUNNING) {
+        cc->reason = why;
+        if (owner) st->reason = why;
+        run = 0;
+      }
     }
-    *run_s = run;
-    *scal_s = scal;
+    cc->run = run;
+    cc->scal = scal;
   }
-  __syncthreads();
+  return consumer_sync(q);
 }
 
 // Last instance whose first ring tile is <= t.
@@ -529,16 +600,20 @@ __device__ __forceinline__ bool ring_any(const CgInst& in, const TileCoord& tc, 
                 : ring_tile<LZ, 1, false>(in, tc, k, scal, q, w, lane, acc);
 }
 
-// All iterations (bar: cooperative launch), or the one phase `phase` (bar
-// null: a device without cooperative launch).
+// All iterations (bar: cooperative launch), or the one phase `phase` (bar.count
+// null: a device without cooperative launch).  Within a phase the producer
+// only follows the ring, so its loads start while the consumers still sum the
+// partials; it skips the tiles of instances that had ended before the phase,
+// and the consumers drain those of an instance that ends at its start.
 __global__ void __launch_bounds__(CR_THREADS, 2)
-    cg_ring(const CgInst* __restrict__ tab, int ninst, int ntiles, CgGrid* bar, int phase) {
+    cg_ring(const CgInst* __restrict__ tab, int ninst, int ntiles, CgGrid bar, int phase) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ double red[32];
-  __shared__ double part[2][CR_WARPS];
-  __shared__ double scal_s;
-  __shared__ int run_s;
+  __shared__ double red[CR_WARPS], part[2][CR_WARPS];
+  __shared__ CgCache cc;
+  __shared__ CgTile pt;  // the producer's
+  __shared__ int slots_s[CR_NA], ok_s;
   unsigned char* base = smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u);
+  volatile int* slots = slots_s;
   CgPipe q;
   q.hd = reinterpret_cast<CgHeader*>(base);
   q.abort_flag = reinterpret_cast<volatile int*>(base + kAbortFlagOffset);
@@ -550,72 +625,145 @@ __global__ void __launch_bounds__(CR_THREADS, 2)
       mbar_init(&q.hd->full[s], 1);
       mbar_init(&q.hd->empty[s], CR_WARPS);
     }
+    mbar_init(&q.hd->sync, CR_WARPS);
     *q.abort_flag = 0;
     q.abort_flag[1] = (int)kCgWaitBudget;
     lg->armedA = lg->parA = lg->armedB = lg->parB = 0;
+    cc.inst = -1;
+    pt.t = -1;
+    cc.run = 1;
     mbar_fence_init();
   }
   __syncthreads();
+  const bool coop = bar.count != nullptr;
   int npart = 0;
+  unsigned int nsync = 0;
   for (;; ++phase) {
     const bool update = phase & 1;
     const int k = phase >> 1;
-    if (update && bar != nullptr) {
+    if (update && coop && ninst > 1) {
       // reasons change in apply phases only: the same answer in every block
       int any = 0;
       for (int i = threadIdx.x; i < ninst; i += CR_THREADS)
         any |= __ldcg(&tab[i].st->reason) == SW_CG_RUNNING;
       if (!__syncthreads_or(any)) break;
     }
-    int cur = -1;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      const int ii = find_ring(tab, ninst, t);
-      const CgInst& in = tab[ii];
-      const int local = t - in.ring_base;
-      if (ii != cur) {
-        __syncthreads();
-        cg_phase_begin(in, update, k, in.ring_base % (int)gridDim.x == (int)blockIdx.x, red,
-                       &run_s, &scal_s);
-        cur = ii;
-      }
-      if (!run_s) continue;
-      const CgRing* rg = reinterpret_cast<const CgRing*>(in.ap);
-      const int lz = rg->lz;
-      const TileCoord tc = tile_coord_t(in.g, rg->tr, local, lz, 512 / lz);
-      if (warp == CR_WARPS) {
-        if (lane == 0 && !*q.abort_flag) {
-          if (update) ring_load<true>(rg, tc, k, q, lg);
-          else ring_load<false>(rg, tc, k, q, lg);
+    if (warp == CR_WARPS) {
+      if (lane == 0) {
+        bool ok = true;
+        for (int t = blockIdx.x; t < ntiles && ok && !*q.abort_flag; t += gridDim.x) {
+          if (t != pt.t) {  // look the tile up
+            const CgInst& in = tab[find_ring(tab, ninst, t)];
+            const CgRing* rg = reinterpret_cast<const CgRing*>(in.ap);
+            pt.rg = rg;
+            pt.st = in.st;
+            pt.t = t;
+            pt.lz = rg->lz;
+            pt.tc = tile_coord_t(in.g, rg->tr, t - in.ring_base, pt.lz, 512 / pt.lz);
+            for (const CUtensorMap* m : {&rg->ph[0], &rg->ph[1], &rg->rh, &rg->rp, &rg->xp})
+              prefetch_tmap(m);
+          }
+          // (a single instance runs until every block leaves)
+          if ((ninst > 1 || !coop) && __ldcg(&pt.st->reason) != SW_CG_RUNNING) continue;
+          ok = update ? ring_load<true>(pt.rg, pt.tc, t, pt.lz, k, q, lg, slots)
+                      : ring_load<false>(pt.rg, pt.tc, t, pt.lz, k, q, lg, slots);
         }
-        __syncwarp();
-      } else if (!*q.abort_flag) {
+        // the end of the phase: one stage armed without a copy
+        if (ok && ws_wait(&q.hd->empty[q.a.s], q.a.ph ^ 1u, q.abort_flag)) {
+          slots[q.a.s] = -1;
+          mbar_arrive(&q.hd->full[q.a.s]);
+          q.a.next();
+        }
+      }
+      __syncwarp();
+    } else {
+      bool fresh = false;  // cc.run and cc.scal are this phase's
+      if (coop && ntiles <= (int)gridDim.x && cc.inst >= 0) {
+        // the block stays with its tile: sum the partials while its first
+        // unit is on the way
+        if (cg_phase_begin(&cc, update, k,
+                           cc.in.ring_base % (int)gridDim.x == (int)blockIdx.x, red, q))
+          fresh = true;
+      }
+      while (true) {
+        if (!ws_wait(&q.hd->full[q.a.s], q.a.ph, q.abort_flag)) break;
+        const int t = slots[q.a.s];
+        if (t < 0) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&q.hd->empty[q.a.s]);
+          q.a.next();
+          break;
+        }
+        const int ii = find_ring(tab, ninst, t);
+        if (!fresh || ii != cc.inst) {
+          if (!consumer_sync(q)) break;
+          if (ii != cc.inst) {
+            const CgRing* rg = reinterpret_cast<const CgRing*>(tab[ii].ap);
+            constexpr int NW = (int)(sizeof(CgInst) / 4);
+            for (int e = threadIdx.x; e < NW; e += CR_CTHREADS)
+              reinterpret_cast<int*>(&cc.in)[e] = reinterpret_cast<const int*>(&tab[ii])[e];
+            if (threadIdx.x == 0) {
+              const CgState* st = tab[ii].st;
+              cc.tr = rg->tr;
+              cc.lz = rg->lz;
+              // (in the first apply phase rs[0] stands in for the one before)
+              cc.rs = __ldcg(&st->rs[update || k == 0 ? (k & 1) : ((k - 1) & 1)]);
+              cc.rs0 = __ldcg(&st->rs0);
+              cc.tol = __ldcg(&st->tol);
+              cc.reason = __ldcg(&st->reason);
+              cc.brk = __ldcg(&st->brk);
+              cc.max_iters = __ldcg(&st->max_iters);
+            }
+            if (!consumer_sync(q)) break;
+            if (threadIdx.x == 0) cc.inst = ii;
+          }
+          if (!cg_phase_begin(&cc, update, k,
+                              cc.in.ring_base % (int)gridDim.x == (int)blockIdx.x, red, q))
+            break;
+          fresh = true;
+        }
+        const int lz = cc.lz, local = t - cc.in.ring_base;
+        const TileCoord tc = tile_coord_t(cc.in.g, cc.tr, local, lz, 512 / lz);
+        if (!cc.run) {  // ended at the start of this phase: drain the tile
+          bool ok = true;
+          for (int u = (tc.x1 - tc.x0 + 1) / 2 + 2; u > 0 && ok; --u) {
+            ok = ws_wait(&q.hd->full[q.a.s], q.a.ph, q.abort_flag);
+            if (!ok) break;
+            if (lane == 0) mbar_arrive(&q.hd->empty[q.a.s]);
+            if (update && u <= (tc.x1 - tc.x0 + 1) / 2) q.next_points();
+            q.a.next();
+          }
+          if (!ok) break;
+          continue;
+        }
         double acc = 0.0;
-        const bool ok = lz == 32 ? ring_any<32>(in, tc, k, update, scal_s, q, warp, lane, &acc)
-                                 : ring_any<64>(in, tc, k, update, scal_s, q, warp, lane, &acc);
+        const bool ok = lz == 32
+                            ? ring_any<32>(cc.in, tc, k, update, cc.scal, q, warp, lane, &acc)
+                            : ring_any<64>(cc.in, tc, k, update, cc.scal, q, warp, lane, &acc);
+        if (!ok) break;
         acc = warp_sum(acc);
         if (lane == 0) part[npart & 1][warp] = acc;
-        // consumers only; a warp that gave up arrives too, so nobody waits for it
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * CR_WARPS) : "memory");
-        if (threadIdx.x == 0 && ok) {
+        if (!consumer_sync(q)) break;
+        if (threadIdx.x == 0) {
           double v = 0.0;
+#pragma unroll
           for (int w = 0; w < CR_WARPS; ++w) v += part[npart & 1][w];
-          reinterpret_cast<double*>(in.partials)[2 * local + (update ? 1 : 0)] = v;
+          cg_partials(cc.in, update)[local] = v;
         }
-        ++npart;
-      } else {
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * CR_WARPS) : "memory");
         ++npart;
       }
     }
-    __syncthreads();
-    if (*q.abort_flag) break;
-    if (bar == nullptr || !cg_grid_sync(bar)) break;
+    if (!coop) break;
+    // a single instance ends in every block alike; the owner has recorded why
+    // (a breakdown found in an update phase ends the next apply phase)
+    if (!cg_grid_sync(bar, ++nsync, q.abort_flag, &ok_s)) break;
+    if (ninst == 1 && !update && !cc.run) break;
   }
   __syncthreads();
   if (*q.abort_flag && warp == CR_WARPS && lane == 0) {
     // let every copy still in flight land, then end the other blocks' waits
     drain_ring(q.hd->full, lg->armedA, lg->parA, CR_NA);
-    if (bar != nullptr) atomicExch(&bar->error, 1);
+    if (coop) atomicOr(bar.gen, kCgGridError);
     else if (ninst > 0) atomicExch(&tab[0].st->brk, -1);
   }
 }
@@ -748,7 +896,7 @@ static int cg_begin(CgInst* in, int base, int* ntiles, cudaStream_t s) {
   const uint64_t dims[3] = {(uint64_t)g.pz, (uint64_t)g.ny, (uint64_t)g.nx};
   const uint64_t strides[2] = {(uint64_t)g.pz * 8, (uint64_t)g.sxy * 8};
   const uint32_t lz = (uint32_t)rg.lz, ly = 512 / lz;
-  const uint32_t halo[3] = {lz + 4, ly + 4, 1}, point[3] = {lz, ly, 1};
+  const uint32_t halo[3] = {lz + 4, ly + 4, 2}, point[3] = {lz, ly, 2};
   struct {
     CUtensorMap* map;
     double* base;
@@ -783,7 +931,7 @@ static int cg_coop_blocks() {
 }
 
 int cg_run(const CgInst* d_tab, int ninst, int ntiles, CgState* d_states, int nst,
-           CgGrid* d_grid, cudaStream_t s) {
+           CgGrid grid_words, cudaStream_t s) {
   if (ntiles == 0) return SW_OK;  // no interior cell
   // One cooperative launch runs every iteration (grid barriers between the
   // phases); without cooperative launch support, phases are launched in
@@ -791,22 +939,24 @@ int cg_run(const CgInst* d_tab, int ninst, int ntiles, CgState* d_states, int ns
   cudaError_t e = cudaFuncSetAttribute(cg_ring, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)CR_SMEM);
   if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(CG smem)");
-  const int coop = d_grid != nullptr ? cg_coop_blocks() : 0;
+  const int coop = cg_coop_blocks();
   if (coop > 0) {
     const int grid = std::max(1, std::min(ntiles, coop));
-    e = cudaMemsetAsync(d_grid, 0, sizeof(CgGrid), s);
+    e = cudaMemsetAsync(grid_words.count, 0, sizeof(unsigned int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(grid_words.gen, 0, sizeof(unsigned int), s);
     int phase = 0;
-    void* args[] = {(void*)&d_tab, (void*)&ninst, (void*)&ntiles, (void*)&d_grid, (void*)&phase};
+    void* args[] = {(void*)&d_tab, (void*)&ninst, (void*)&ntiles, (void*)&grid_words,
+                    (void*)&phase};
     if (e == cudaSuccess)
       e = cudaLaunchCooperativeKernel((const void*)cg_ring, dim3(grid), dim3(CR_THREADS), args,
                                       CR_SMEM, s);
     if (e != cudaSuccess) return cuda_status(e, "cg_ring launch");
     count_launches(1);
-    CgGrid hg{};
-    e = cudaMemcpyAsync(&hg, d_grid, sizeof(hg), cudaMemcpyDeviceToHost, s);
+    unsigned int gen = 0;
+    e = cudaMemcpyAsync(&gen, grid_words.gen, sizeof(gen), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e, "cg_ring readback");
-    if (hg.error) {
+    if (gen & kCgGridError) {
       set_error("CG: a bounded wait of the persistent kernel ran out");
       return SW_ETIMEOUT;
     }
@@ -831,7 +981,7 @@ int cg_run(const CgInst* d_tab, int ninst, int ntiles, CgState* d_states, int ns
     }
     if (!running) return SW_OK;
     for (int b = 0; b < batch; ++b, ++phase)
-      cg_ring<<<grid, CR_THREADS, CR_SMEM, s>>>(d_tab, ninst, ntiles, nullptr, phase);
+      cg_ring<<<grid, CR_THREADS, CR_SMEM, s>>>(d_tab, ninst, ntiles, CgGrid{}, phase);
     count_launches((unsigned long long)batch);
     SW_CHECK_LAUNCH("cg iteration");
     batch = std::min(batch * 2, 128);
@@ -1037,7 +1187,7 @@ BatchTableLayout batch_layout(int n) {
   L.outs = off;
   off += align_up((size_t)n * sizeof(double*), 256);
   L.grid = off;
-  off += align_up(sizeof(CgGrid), 256);
+  off += 256;  // cg_grid_at
   L.total = off;
   return L;
 }
@@ -1103,7 +1253,7 @@ int project_batch_t(const sw_project_job* jobs, int n, char* table, sw_cg_stats*
                                                      (const InStride*)(table + L.strides));
     count_launches(1);
     SW_CHECK_LAUNCH("cg_prep (batch)");
-    int rc = cg_run(d_tab, n, nring, d_states, n, (CgGrid*)(table + L.grid), s);
+    int rc = cg_run(d_tab, n, nring, d_states, n, cg_grid_at(table + L.grid), s);
     if (rc != SW_OK) return rc;
     cg_finish<T><<<grid, dim3(TILE_Z, TILE_Y), 0, s>>>(d_tab, n, ntiles,
                                                        (const T* const*)(table + L.fin),

@@ -24,18 +24,21 @@ struct CgState {
   unsigned int ticket;
 };
 
-static_assert(sizeof(CgState) <= 128, "the grid barrier shares the state's 256-byte slot");
-
-// Grid-wide barrier of the persistent CG kernel (zeroed before each launch):
-// arrivals, generation, and an error word set when a wait runs out.
+// Grid-wide barrier of the persistent CG kernel: a count of arrivals and the
+// number of the last barrier passed, 128-byte lines apart, both zeroed before
+// each launch.  The top bit of `gen` is set when a wait runs out.
 struct CgGrid {
-  unsigned int count;
-  unsigned int gen;
-  int error;
-  int pad;
+  unsigned int* count;
+  unsigned int* gen;
 };
-// The barrier of a single solve lives 128 bytes after its state.
-inline CgGrid* cg_grid_of(CgState* st) { return (CgGrid*)((char*)st + 128); }
+constexpr unsigned int kCgGridError = 0x80000000u;
+// In a 256-byte block of its own (a batch), or in a single solve's 256-byte
+// state block: `gen` after the state, `count` in the second line.
+inline CgGrid cg_grid_at(char* block) {
+  return CgGrid{(unsigned int*)(block + 128), (unsigned int*)(block + 120)};
+}
+static_assert(sizeof(CgState) <= 120, "the grid barrier shares the state's 256-byte slot");
+inline CgGrid cg_grid_of(CgState* st) { return cg_grid_at((char*)st); }
 
 // One solve in a launch's instance table.
 //   op 0: the projection's Poisson operator A = -div_c(grad_c .)

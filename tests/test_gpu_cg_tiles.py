@@ -52,3 +52,27 @@ def test_static_solve_at_tile_edges(cuda, shape, field):
     ref = O.elastic_solve_static(b, *h, mu, tol=tol, max_iters=iters, dtype=np.float64)
     out = sw.elastic_solve_static(b, *h, mu, tol=tol, max_iters=iters, info=info)
     assert _rel(out, ref) <= 1e-7, info
+
+
+def test_batched_projection_with_ended_and_tiny_instances(cuda):
+    """Instances that need no iteration, that stop early and that run long share a
+    launch; each gives the bits of its own run."""
+    import torch
+
+    import shearwave_b200 as sw
+    from shearwave_b200 import ops
+
+    rng = np.random.default_rng(5)
+    shapes = [(12, 11, 10), (3, 3, 3), (40, 33, 70), (9, 18, 34), (2, 5, 6), (33, 34, 66)]
+    h, tols, iters = 0.5e-3, [1e-9, 1e-9, 1e-9, 1e-3, 1e-9, 1e-9], [500, 500, 500, 500, 500, 4]
+    f = [[torch.as_tensor(rng.standard_normal(s), device=cuda) for _ in range(3)] for s in shapes]
+    f[3] = [torch.zeros_like(c) for c in f[3]]  # divergence-free: early exit
+    outs, stats = ops.project_batch([c[0] for c in f], [c[1] for c in f], [c[2] for c in f],
+                                    [h] * 18, tols, iters)
+    for k, s in enumerate(shapes):
+        info = {}
+        alone = sw.project_vector_field(*f[k], h, h, h, tols[k], iters[k], info=info)
+        pz = ops.pitch(s[2])
+        both = outs[k].reshape(3, s[0], s[1], pz)[..., :s[2]]
+        assert all(torch.equal(a, b) for a, b in zip(alone, both)), k
+        assert int(stats[k, 0]) == info["iters"]
