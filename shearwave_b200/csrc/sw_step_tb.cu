@@ -455,13 +455,68 @@ __device__ __forceinline__ TbPos tb_tile_sw(const TmaF32TB* __restrict__ in, int
 }
 
 
+// Progress of a resident launch's tiles: `words` holds one count per tile,
+// `stride` words apart, of the consumer warps that have finished it (15 per
+// pair of steps).
+struct TbProgress {
+  int* words;
+  int stride, npairs;
+};
+
+// End of a block of a resident launch (every thread): the last one to finish
+// clears the progress words and the finish count.
+__device__ __forceinline__ void tb_resident_done(int* queues, const TbProgress& pr, int ntiles) {
+  __shared__ int last_s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last_s = atomicAdd(queues + 1, 1) == (int)gridDim.x - 1;
+    if (last_s) atomicExch(queues + 1, 0);
+  }
+  __syncthreads();
+  if (last_s)
+    for (int t = threadIdx.x; t < ntiles; t += blockDim.x) pr.words[t * pr.stride] = 0;
+}
+
+// Whole producer warp: wait until tile `t` and the tiles around it have
+// finished `need` warps' work.  Bounded like ws_wait; gives up as soon as the
+// solve is abandoned (returns false, the block ends its work).
+__device__ __forceinline__ bool tb_wait_around(const TmaF32TB& in, const TbProgress& pr, int t,
+                                               int need, volatile int* abort_flag, int lane) {
+  const TileSpace& ts = in.ts;
+  const int zt = t % ts.ntz + lane % 3 - 1, yt = t / ts.ntz % ts.nty + lane / 3 % 3 - 1,
+            xt = t / ts.ntz / ts.nty + lane / 9 - 1;
+  const bool mine = lane < 27 && zt >= 0 && zt < ts.ntz && yt >= 0 && yt < ts.nty && xt >= 0 &&
+                    xt < ts.nxc;
+  const int* w = pr.words + (mine ? ((xt * ts.nty + yt) * ts.ntz + zt) * pr.stride : 0);
+  const uint32_t t0 = (uint32_t)clock();
+  while (true) {
+    int v = need;
+    if (mine) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(w) : "memory");
+    if (__all_sync(0xffffffffu, v >= need)) return true;
+    const bool late = (((uint32_t)clock() - t0) >> 10) > (uint32_t)abort_flag[1];
+    if (late) *abort_flag = 1;
+    if (__any_sync(0xffffffffu, late || *abort_flag != 0 || solve_abandoned(in.flags)))
+      return false;
+  }
+}
+
 // LZ 0 (batched launches): each solve's tiles have the solve's own shape
 // (TmaF32TB::lz), the one that computes fewer cells on its grid.
-template <bool BATCH, int LZ>
+//
+// RES (a lone solve, cooperative launch): the blocks stay for pr.npairs pairs
+// of steps, each with its own tiles, and a tile starts its next pair as soon
+// as the tiles around it have finished the one before (their halos are
+// written; with three state buffers nobody still reads the one it writes), so
+// the launches, barrier set-ups and pipeline fills between pairs, and the wait
+// for the slowest tile of the grid, are gone.
+template <bool BATCH, int LZ, bool RES = false>
 __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
     step_f32_fused2(const __grid_constant__ TmaF32TB one, const TmaF32TB* __restrict__ tab,
-                    int ninst, int ntiles, int it, const int* __restrict__ it_dev, int* queues) {
+                    int ninst, int ntiles, int it, const int* __restrict__ it_dev, int* queues,
+                    TbProgress pr) {
   static_assert(LZ != 0 || BATCH, "a single solve has one shape");
+  static_assert(!RES || !BATCH, "a resident launch is a lone solve's");
   if (it_dev != nullptr) it += *it_dev;  // step counter kept on the device (graph replays)
   // batched launches take tiles from a launch-wide queue (see step_f32_tma)
   int* queue = queues;
@@ -483,7 +538,8 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
     if (threadIdx.x == 0)
       for (int k = 0; k < (BATCH ? ninst : 1); ++k)
         if (int* fl = flags_of(k)) atomicOr(fl, kFlagRefused);
-    queue_cta_done(queue);
+    if (RES) tb_resident_done(queue, pr, ntiles);
+    else queue_cta_done(queue);
     return;
   }
   AbortLog* lg = abort_log(base);
@@ -504,18 +560,103 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
 
   if (warp == T::CONSUMER_WARPS) {
     // ------------------------------- producer -----------------------------
-    if (lane == 0) {
-      RingPos<NA> pa;
-      RingPos<NB> pb;
+    RingPos<NA> pa;
+    RingPos<NB> pb;
+    bool ok = true;
+    // one lane: the planes of one tile (`tag` goes to the consumers with it)
+    auto load_tile = [&](const T* in, int k, int tag, int t, int local, int lit, bool push) {
+      const int ord = lg->n_taken;  // the tile's ordinal: its term buffer
+      lg->solve[lg->n_taken & 7] = k;
+      ++lg->n_taken;
+      const Geom& g = in->g;
+      const TbDims dm = LZ == 32 || (LZ == 0 && in->lz == 32) ? tb_dims<32>() : tb_dims<64>();
+      const TbCoord tc = tb_coord_rt(g, in->ts, local, dm.oz, dm.oy);
+      const CUtensorMap* tma = &in->tm[lit % 3];
+      const uint32_t bbytes = dm.b_cells * 4 * in->ncoef;
+      bool first = true;
+      // level-0 plane p, and from plane x0 on the coefficients of plane p-1
+      // (what level 1 of plane p-1 reads) on the same barrier
+      auto issue = [&](int p) {
+        const int sa = pa.s;
+        ok = ok && ws_wait(&hd->emptyA[sa], pa.ph ^ 1u, abort_flag);
+        if (!ok) return;
+        if (first) {
+          first = false;
+          if (in->stall_test) {  // the testing switch leaves the tile's first stage unarmed
+            pa.next();
+            return;
+          }
+          tile_slots(base)[sa] = t;
+          solve_slots(base)[sa] = tag;
+          if (push) {  // every warp has left tile ord-2, which used this buffer
+            TbTermBuf& tb = terms[ord & 1];
+            const unsigned nc = (unsigned)g.ncell;
+            for (int lev = 0; lev < 2; ++lev) {
+              const int j0 = in->term_off[lit + lev], j1 = in->term_off[lit + lev + 1];
+              tb.n[lev] = j1 - j0;
+              for (int j = j0; j < j1; ++j)
+                tb.t[lev][j - j0] = TbTermRef{in->pat + (long long)in->term_pat[j] * 3 * nc,
+                                              (float)in->term_scale[j], 0};
+            }
+          }
+        }
+        const int pl = min(max(p, 0), g.nx - 1);  // planes outside the grid feed only the shell
+        fence_proxy_async_smem();
+        const bool points = p >= tc.x0;
+        mbar_arrive_expect_tx(&hd->fullA[sa], dm.a_bytes + (points ? bbytes : 0u));
+        tma_load_4d(ringA + sa * AF, tma, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 2, pl, 0);
+        if (points) {
+          const int ql = min(max(p - 1, 0), g.nx - 1);
+          tma_load_4d(ringB + pb.s * BF, &in->tmm, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 1, ql, 0);
+          pb.next();
+        }
+        arm_record(lg->armedA, lg->parA, sa, pa.ph);
+        pa.next();
+      };
+      for (int p = tc.x0 - 2; p <= tc.x1 + 1 && ok; ++p) issue(p);
+    };
+    // whether a pair's force terms fit the term buffer (see kTbTermCap)
+    auto terms_fit = [&](const T* in, int lit) -> bool {
+      return in->term_off[lit + 1] - in->term_off[lit] <= kTbTermCap &&
+             in->term_off[lit + 2] - in->term_off[lit + 1] <= kTbTermCap;
+    };
+    auto end_work = [&]() {  // arm one stage without a copy
+      if (!ws_wait(&hd->emptyA[pa.s], pa.ph ^ 1u, abort_flag)) return;
+      tile_slots(base)[pa.s] = -1;
+      mbar_arrive(&hd->fullA[pa.s]);
+      pa.next();
+    };
+    if (RES) {
+      bool go = true;
+      for (int j = 0; j < pr.npairs && go; ++j) {
+        const int lit = it + 2 * j;
+        for (int t = blockIdx.x; t < ntiles && go; t += gridDim.x) {
+          if (j > 0)
+            go = tb_wait_around(one, pr, t, j * T::CONSUMER_WARPS, abort_flag, lane);
+          else
+            go = !solve_abandoned(one.flags);
+          go = __all_sync(0xffffffffu, go);
+          if (!go) break;
+          if (lane == 0) {
+            fence_proxy_async_all();  // the neighbours' stores before this tile's copies
+            const bool push = tb_pushes(&one, lit);
+            if (push && !terms_fit(&one, lit)) {
+              if (one.flags != nullptr) atomicOr(one.flags, kFlagRefused);
+              ok = false;
+            } else {
+              load_tile(&one, 0, j, t, t, lit, push);
+            }
+          }
+          go = __all_sync(0xffffffffu, ok) && !*abort_flag;
+        }
+      }
+      if (lane == 0 && !*abort_flag) end_work();
+    } else if (lane == 0) {
       int stride_next = blockIdx.x;
-      bool ok = true;
       while (ok && !*abort_flag) {
         const int t = next_tile(queue, stride_next);
-        if (t >= ntiles) {  // end of this CTA's work: arm one stage without a copy
-          if (!ws_wait(&hd->emptyA[pa.s], pa.ph ^ 1u, abort_flag)) break;
-          tile_slots(base)[pa.s] = -1;
-          mbar_arrive(&hd->fullA[pa.s]);
-          pa.next();
+        if (t >= ntiles) {
+          end_work();
           break;
         }
         const int k = BATCH ? find_solve(tab, ninst, t) : 0;
@@ -524,60 +665,11 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
         const int lit = it - in->it_begin;
         if (lit < 0 || lit + 1 >= in->n_steps || solve_abandoned(in->flags)) continue;
         const bool push = tb_pushes(in, lit);
-        if (push && (in->term_off[lit + 1] - in->term_off[lit] > kTbTermCap ||
-                     in->term_off[lit + 2] - in->term_off[lit + 1] > kTbTermCap)) {
-          if (in->flags != nullptr) atomicOr(in->flags, kFlagRefused);  // see kTbTermCap
+        if (push && !terms_fit(in, lit)) {
+          if (in->flags != nullptr) atomicOr(in->flags, kFlagRefused);
           continue;
         }
-        const int ord = lg->n_taken;  // the tile's ordinal: its term buffer
-        lg->solve[lg->n_taken & 7] = k;
-        ++lg->n_taken;
-        const Geom& g = in->g;
-        const TbDims dm = LZ == 32 || (LZ == 0 && in->lz == 32) ? tb_dims<32>() : tb_dims<64>();
-        const TbCoord tc = tb_coord_rt(g, in->ts, local, dm.oz, dm.oy);
-        const CUtensorMap* tma = &in->tm[lit % 3];
-        const uint32_t bbytes = dm.b_cells * 4 * in->ncoef;
-        bool first = true;
-        // level-0 plane p, and from plane x0 on the coefficients of plane p-1
-        // (what level 1 of plane p-1 reads) on the same barrier
-        auto issue = [&](int p) {
-          const int sa = pa.s;
-          ok = ok && ws_wait(&hd->emptyA[sa], pa.ph ^ 1u, abort_flag);
-          if (!ok) return;
-          if (first) {
-            first = false;
-            if (in->stall_test) {  // the testing switch leaves the tile's first stage unarmed
-              pa.next();
-              return;
-            }
-            tile_slots(base)[sa] = t;
-            solve_slots(base)[sa] = k;
-            if (push) {  // every warp has left tile ord-2, which used this buffer
-              TbTermBuf& tb = terms[ord & 1];
-              const unsigned nc = (unsigned)g.ncell;
-              for (int lev = 0; lev < 2; ++lev) {
-                const int j0 = in->term_off[lit + lev], j1 = in->term_off[lit + lev + 1];
-                tb.n[lev] = j1 - j0;
-                for (int j = j0; j < j1; ++j)
-                  tb.t[lev][j - j0] = TbTermRef{in->pat + (long long)in->term_pat[j] * 3 * nc,
-                                                (float)in->term_scale[j], 0};
-              }
-            }
-          }
-          const int pl = min(max(p, 0), g.nx - 1);  // planes outside the grid feed only the shell
-          fence_proxy_async_smem();
-          const bool points = p >= tc.x0;
-          mbar_arrive_expect_tx(&hd->fullA[sa], dm.a_bytes + (points ? bbytes : 0u));
-          tma_load_4d(ringA + sa * AF, tma, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 2, pl, 0);
-          if (points) {
-            const int ql = min(max(p - 1, 0), g.nx - 1);
-            tma_load_4d(ringB + pb.s * BF, &in->tmm, &hd->fullA[sa], tc.z0 - 4, tc.y0 - 1, ql, 0);
-            pb.next();
-          }
-          arm_record(lg->armedA, lg->parA, sa, pa.ph);
-          pa.next();
-        };
-        for (int p = tc.x0 - 2; p <= tc.x1 + 1 && ok; ++p) issue(p);
+        load_tile(in, k, k, t, local, lit, push);
       }
     }
   } else {
@@ -591,7 +683,7 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
       if (t < 0) break;
       const T* in = BATCH ? &tab[solve_slots(base)[p.ca.s]] : &one;
       const int local = BATCH ? t - in->tile_base : t;
-      const int lit = it - in->it_begin;
+      const int lit = RES ? it + 2 * solve_slots(base)[p.ca.s] : it - in->it_begin;
       if (LZ == 0)
         p = in->lz == 32 ? tb_tile_sw<32>(in, local, lit, k, p, warp, lane)
                          : tb_tile_sw<64>(in, local, lit, k, p, warp, lane);
@@ -600,6 +692,13 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
       if (!p.ok) break;
       ++p.ord;
       if (lane == 0) ++lg->done[warp];
+      if (RES) {  // this warp's rows of the tile are written
+        fence_proxy_async_all();
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(pr.words + t * pr.stride)
+                       : "memory");
+      }
     }
   }
   __syncthreads();
@@ -607,8 +706,11 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
     // let every copy still in flight land, then flag the abandoned tiles' solves
     drain_ring(hd->fullA, lg->armedA, lg->parA, NA);
     flag_unfinished(lg, T::CONSUMER_WARPS, BATCH ? ninst : 1, kFlagTimeout, flags_of);
+    // (a wait for other tiles leaves none of this block's own unfinished)
+    if (RES && one.flags != nullptr) atomicOr(one.flags, kFlagTimeout);
   }
-  queue_cta_done(queue);
+  if (RES) tb_resident_done(queue, pr, ntiles);
+  else queue_cta_done(queue);
 }
 
 }  // namespace
@@ -628,11 +730,13 @@ static int tb_set_attr() {
   static bool done = false;
   if (done) return SW_OK;
   const int bytes = (int)tb_smem_bytes();
-  const void* fns[5] = {(const void*)step_f32_fused2<false, 64>,
+  const void* fns[7] = {(const void*)step_f32_fused2<false, 64>,
                         (const void*)step_f32_fused2<true, 64>,
                         (const void*)step_f32_fused2<false, 32>,
                         (const void*)step_f32_fused2<true, 32>,
-                        (const void*)step_f32_fused2<true, 0>};
+                        (const void*)step_f32_fused2<true, 0>,
+                        (const void*)step_f32_fused2<false, 64, true>,
+                        (const void*)step_f32_fused2<false, 32, true>};
   for (const void* f : fns) {
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(fused step smem)");
@@ -758,9 +862,69 @@ const void* step_f32_fused2_batch_ptr(int lz) {
 static void launch_tb(const void* fn, int grid, cudaStream_t s, const TmaF32TB& one,
                       const TmaF32TB* tab, int ninst, int ntiles, int it, int* queues) {
   const int* itd = nullptr;
+  TbProgress none{};
   void* args[] = {(void*)&one, (void*)&tab, (void*)&ninst, (void*)&ntiles, (void*)&it,
-                  (void*)&itd, (void*)&queues};
+                  (void*)&itd, (void*)&queues, (void*)&none};
   cudaLaunchKernel(fn, dim3(grid), dim3(TmaF32TB::THREADS), args, tb_smem_bytes(), s);
+}
+
+// SMs a cooperative launch of the resident kernel can use on the current
+// device, or 0 when it cannot run one block per SM.
+static int tb_resident_slots(int lz) {
+  int dev = 0, coop = 0, sms = 0, per = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+    return 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  const void* fn = lz == 32 ? (const void*)step_f32_fused2<false, 32, true>
+                            : (const void*)step_f32_fused2<false, 64, true>;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, TmaF32TB::THREADS,
+                                                    tb_smem_bytes()) != cudaSuccess)
+    return 0;
+  return per * sms;
+}
+
+// Run pairs of a lone solve in resident launches (prepared: tb_set_attr).  The
+// progress words lie in the shell plane x = 0 of the compensation component of
+// state buffer 0, which is zero in every state and is cleared again, so the
+// solve's own memory carries them: any number of solves, streams and threads.
+// A launch holds the GPU until it ends, so it is bounded to about 2 ms of work
+// (between 16 and 512 pairs).  *done: steps enqueued, 0 when the solve's tiles
+// do not allow it.
+int run_fused2_resident(const TmaF32TB& t, int* queue, int it0, int nsteps, cudaStream_t s,
+                        int* done, unsigned long long* launches) {
+  *done = 0;
+  const int pairs = nsteps / 2, ntiles = t.ts.count;
+  // (chunks of one plane would reach past their neighbours)
+  if (queue == nullptr || pairs < 2 || ntiles == 0 || (t.ts.xc < 2 && t.ts.nxc > 1)) return SW_OK;
+  const int stride = (int)std::min<long long>(8, t.g.sxy / ntiles);
+  if (stride < 1) return SW_OK;
+  const int slots = tb_resident_slots(t.lz);
+  if (slots == 0) return SW_OK;
+  const int grid = std::min(ntiles, slots);
+  TbProgress pr{reinterpret_cast<int*>(t.state[0] + 6 * t.g.ncell), stride, 0};
+  const long long cells = (long long)t.g.nx * t.g.ny * t.g.nz;
+  const int most = (int)std::max<long long>(16, std::min<long long>(512, 100000000LL / cells));
+  const void* fn = t.lz == 32 ? (const void*)step_f32_fused2<false, 32, true>
+                              : (const void*)step_f32_fused2<false, 64, true>;
+  const TmaF32TB* tab = nullptr;
+  const int* itd = nullptr;
+  int ninst = 1, nt = ntiles;
+  cudaError_t e = cudaMemsetAsync(pr.words, 0, sizeof(int) * (size_t)ntiles * stride, s);
+  for (int left = pairs; left > 0 && e == cudaSuccess; left -= pr.npairs) {
+    // equal launches
+    const int n = (left + most - 1) / most;
+    pr.npairs = (left + n - 1) / n;
+    int it = it0 + *done;
+    void* args[] = {(void*)&t,   (void*)&tab,   (void*)&ninst, (void*)&nt,
+                    (void*)&it, (void*)&itd, (void*)&queue, (void*)&pr};
+    e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(TmaF32TB::THREADS), args, tb_smem_bytes(),
+                                    s);
+    *done += 2 * pr.npairs;
+    ++*launches;
+  }
+  if (e != cudaSuccess) return cuda_status(e, "resident two-step launch");
+  return SW_OK;
 }
 
 void launch_fused2_raw(const TmaF32TB& t, int it, cudaStream_t s) {

@@ -946,10 +946,11 @@ int graph_loop(void* func, const Inst& t, int grid, int threads, size_t smem, in
   const int* itd = clock;
   int* queues = queue;
   std::vector<int> offs(seg);
+  long long none[2] = {};  // the two-step kernels' last argument (unused outside resident launches)
   for (int k = 0; k < seg && e == cudaSuccess; ++k) {
     offs[k] = k * per_launch;
     void* args[] = {(void*)&t,        (void*)&tab, (void*)&ninst, (void*)&ntiles,
-                    (void*)&offs[k], (void*)&itd, (void*)&queues};
+                    (void*)&offs[k], (void*)&itd, (void*)&queues, (void*)&none};
     cudaKernelNodeParams p{};
     p.func = func;
     p.gridDim = dim3(grid);
@@ -1025,14 +1026,20 @@ int launch_steps_tma(const StepArgs& a, int xchunk, int it0, int nsteps, cudaStr
     const int grid = std::min(t.ts.count, step_slots());
     unsigned long long n_launch = 0;
     int done = 0;
-    if (fuse && tb.ts.count > 0)
-      rc = graph_loop(const_cast<void*>(step_f32_fused2_ptr(tb.lz)), tb,
-                      std::min(tb.ts.count, kNumSMs), TmaF32TB::THREADS, tb_smem_bytes(), 2, 16,
-                      a.clock, a.queue, it0, nsteps, s, &done);
-    else
-      rc = graph_loop(const_cast<void*>(f32_kernel(false, t.tzw, t.kahan != 0)), t, grid,
-                      TmaF32::THREADS, f32_smem(t.kahan != 0), 1, 32, a.clock, a.queue, it0,
-                      nsteps, s, &done);
+    // long runs: resident launches of the two-step kernel, else one graph of
+    // launches replayed (a null clock asks for plain launches)
+    if (fuse && tb.ts.count > 0 && a.clock != nullptr)
+      rc = run_fused2_resident(tb, a.queue, it0, nsteps, s, &done, &n_launch);
+    if (rc == SW_OK && done == 0) {
+      if (fuse && tb.ts.count > 0)
+        rc = graph_loop(const_cast<void*>(step_f32_fused2_ptr(tb.lz)), tb,
+                        std::min(tb.ts.count, kNumSMs), TmaF32TB::THREADS, tb_smem_bytes(), 2, 16,
+                        a.clock, a.queue, it0, nsteps, s, &done);
+      else
+        rc = graph_loop(const_cast<void*>(f32_kernel(false, t.tzw, t.kahan != 0)), t, grid,
+                        TmaF32::THREADS, f32_smem(t.kahan != 0), 1, 32, a.clock, a.queue, it0,
+                        nsteps, s, &done);
+    }
     if (rc != SW_OK) return rc;
     for (int it = it0 + done; it < it0 + nsteps;) {
       if (fuse && it + 1 < it0 + nsteps) {

@@ -169,6 +169,10 @@ int make_tma_f32_tb(const StepArgs& a, int xchunk, TmaF32TB* t, int lz);
 int launch_fused2(const StepArgs& a, int xchunk, int it, cudaStream_t s);
 int launch_fused2_prepare();                                   // kernel attributes, once
 void launch_fused2_raw(const TmaF32TB& t, int it, cudaStream_t s);  // enqueue one launch
+// Pairs of a lone solve in resident launches; *done: steps enqueued.
+int run_fused2_resident(const TmaF32TB& t, int* queue, int it0, int nsteps, cudaStream_t s,
+                        int* done, unsigned long long* launches);
+// (in graph nodes the two-step kernels take one argument more, zero)
 const void* step_f32_fused2_ptr(int lz);        // the single-solve fused kernel (graph nodes)
 const void* step_f32_fused2_batch_ptr(int lz);  // the batched fused kernel (graph nodes)
 int launch_fused2_batch(const void* d_tab, int ninst, int ntiles, int it, int* queues, int lz,

@@ -29,6 +29,11 @@ __device__ inline void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Orders generic accesses (global ones included) and asynchronous-proxy ones.
+__device__ inline void fence_proxy_async_all() {
+  asm volatile("fence.proxy.async;" ::: "memory");
+}
+
 // Arrive once (the producer) and announce `bytes` of transaction.
 __device__ inline void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
