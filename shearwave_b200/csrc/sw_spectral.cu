@@ -109,18 +109,23 @@ __global__ void axis_basis_kernel(int n, double h, AxisBasis ax) {
 // ---------------------------------------------------------------------------
 // A basis couples cells of one parity only, so an axis of n cells is two
 // products with matrices of n/2 rows: half the multiply-adds of one n x n
-// product.  What bounds them is the FP64 pipe (64 fused multiply-adds per
-// cycle and SM).  A warp owns 32 modes x 32 data columns, a thread 8 x 4
-// accumulators (six to eight shared-memory wavefronts per 32 multiply-adds
-// of the warp, under half of what the pipe leaves time for), operands come
-// through a three-stage cp.async ring 16 deep.  A block takes WM units of 32
-// modes: a chain of up to 128 modes reads its data once and pads its modes
-// to a multiple of 32 only.  Measured against 64 x 64 tiles of the full
-// n x n matrices with 8-byte loads and no pipeline: the six transforms of a
-// 160 x 131 x 173 grid 1154 -> 339 us (whole projection 1406 -> 523 us), the
-// 48 of eight 256 x 256 x 384 forces 75.4 -> 21.0 ms (axes x and y at 20
-// TFLOP/s of the multiply-adds a chain needs, axis z at 14.5).
+// product.  What bounds them is the FP64 rate (64 multiply-adds per cycle and
+// SM).  A warp owns 32 modes x 32 data columns as 16 m8n8k4 products on the
+// FP64 matrix unit (eight 8-byte shared loads per 16 products; with fused
+// multiply-adds, 8 x 4 accumulators a thread, half the instructions were not
+// multiply-adds), operands come through a three-stage cp.async ring 16 deep.
+// A block takes WM units of 32 modes: a chain of up to 128 modes reads its
+// data once and pads its modes to a multiple of 32 only.  Measured: 64 x 64
+// tiles of the full n x n matrices with 8-byte loads and no pipeline, then
+// multiply-adds on the chains, then this: the six transforms of a 160 x 131 x
+// 173 grid 1154, 339, 246 us (whole projection 1406, 523, 426 us), the 48 of
+// eight 256 x 256 x 384 forces 75.4, 21.0, 15.0 ms (axes x and y at 28
+// TFLOP/s of the multiply-adds a chain needs, axis z at 20).
 constexpr int SG_K = 16, SG_STAGES = 3;
+constexpr int SG_PAD = 8;  // rows 64 bytes apart modulo 128: the four depths of a fragment
+// resident blocks per SM: 16 to 18 warps (a multiply-add's latency is covered
+// by a thread's 32 accumulators; more warps cover the copies and barriers)
+#define SG_BLOCKS(WM) ((WM) == 1 ? 8 : (WM) == 2 ? 4 : (WM) == 3 ? 3 : 2)
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
@@ -140,17 +145,49 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// A warp's 32 (modes) x 32 (data) tile of products for one 16-deep chunk on
+// the FP64 matrix unit: w[b * LDW + mode], data column n of depth b at
+// d[n * dn + b * db].  acc[i][j]: modes 8 i + lane / 4, data 8 j + 2 (lane % 4)
+// and the next.
+template <int LDW>
+__device__ __forceinline__ void mma_chunk(const double* __restrict__ w,
+                                          const double* __restrict__ d, int dn, int db,
+                                          double (&acc)[4][4][2], int lane) {
+  const double* wp = w + (lane & 3) * LDW + (lane >> 2);
+  const double* dp = d + (lane & 3) * db + (lane >> 2) * dn;
+#pragma unroll
+  for (int kk = 0; kk < SG_K; kk += 4) {
+    double a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = wp[kk * LDW + 8 * i];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = dp[kk * db + 8 * j * dn];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+            : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+            : "d"(a[i]), "d"(b[j]));
+  }
+}
+
 // Rows b0 .. b0+15 of a chain's matrix, columns a0 .. a0+32 WM-1 (zero
-// outside the matrix).
-template <int WM, int THREADS>
+// outside the matrix), by the 64 WM threads of a block: a thread keeps its
+// column and copies every other row.
+template <int WM>
 __device__ __forceinline__ void load_w(double* __restrict__ ws, const double* __restrict__ W,
                                        int K, int b0, int a0, int tid) {
-  constexpr int LD = 32 * WM;
-  for (int e = tid; e < SG_K * LD; e += THREADS) {
-    const int kk = e / LD, a = e % LD;
-    const int b = b0 + kk, col = a0 + a;
-    const bool ok = b >= 0 && b < K && col < K;
-    cp_async8(ws + kk * LD + a, ok ? W + (long long)b * K + col : W, ok);
+  constexpr int N = 32 * WM, LD = N + SG_PAD;
+  const int half = tid >= N ? 1 : 0, a = tid - half * N;
+  const bool col = a0 + a < K;
+  const double* src = W + (long long)(b0 + half) * K + a0 + a;
+  double* dst = ws + half * LD + a;
+#pragma unroll
+  for (int kk = 0; kk < SG_K; kk += 2) {
+    const bool ok = col && (unsigned)(b0 + half + kk) < (unsigned)K;
+    cp_async8(dst + kk * LD, ok ? src : W, ok);
+    src += 2 * K;
   }
 }
 
@@ -159,34 +196,39 @@ __device__ __forceinline__ void load_w(double* __restrict__ ws, const double* __
 // run of a whole plane; axis y: the z rows of all interior planes).  nper is
 // even, so the 16-byte pieces never straddle two runs.
 template <int WM>
-__global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
+__global__ void __launch_bounds__(64 * WM, SG_BLOCKS(WM))
     spec_rows(AxisBasis ax, int inverse, const double* __restrict__ src, double* __restrict__ dst,
               long long rs, int nper, long long nstride, long long ntot) {
-  constexpr int THREADS = 64 * WM, LDW = 32 * WM, LDD = 64;
+  constexpr int LDW = 32 * WM + SG_PAD, LDD = 64 + SG_PAD;
   extern __shared__ __align__(16) double smem[];
-  double* wsm = smem;                               // [stage][16][32 WM]
-  double* dsm = smem + SG_STAGES * SG_K * LDW;      // [stage][16][64]
+  double* wsm = smem;                               // [stage][16][32 WM + 8]
+  double* dsm = smem + SG_STAGES * SG_K * LDW;      // [stage][16][64 + 8]
   const int par = blockIdx.z, K = ax.K[par];
-  const int a0 = blockIdx.y * LDW;
+  const int a0 = blockIdx.y * 32 * WM;
   if (a0 >= K) return;
   const double* W = ax.W[inverse][par];
   const long long n0 = blockIdx.x * 64ll;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp % WM, wn = warp / WM, gm = lane >> 3, gn = lane & 7;
+  const int wm = warp % WM, wn = warp / WM;
   const double* base = src + chain_first(par) * rs;
   // pieces of two columns: this thread copies piece tid % 32 of some rows
   const long long pn = n0 + 2 * (tid & 31);
   const bool pok = pn < ntot;
   const long long poff = pok ? (pn / nper) * nstride + pn % nper : 0;
   auto load = [&](int st, int b0) {
-    load_w<WM, THREADS>(wsm + st * SG_K * LDW, W, K, b0, a0, tid);
-    for (int kk = tid >> 5; kk < SG_K; kk += THREADS / 32) {
-      const bool ok = pok && b0 + kk < K;
-      cp_async16(dsm + (st * SG_K + kk) * LDD + 2 * (tid & 31),
-                 ok ? base + 2 * (b0 + kk) * rs + poff : src, ok);
+    load_w<WM>(wsm + st * SG_K * LDW, W, K, b0, a0, tid);
+    const int k0 = tid >> 5;
+    const double* p = base + 2 * (b0 + k0) * rs + poff;
+    double* d = dsm + (st * SG_K + k0) * LDD + 2 * (tid & 31);
+#pragma unroll
+    for (int kk = 0; kk < SG_K; kk += 2 * WM) {
+      if (k0 + kk >= SG_K) break;
+      const bool ok = pok && b0 + k0 + kk < K;
+      cp_async16(d + kk * LDD, ok ? p : src, ok);
+      p += 4ll * WM * rs;
     }
   };
-  double acc[8][4] = {};
+  double acc[4][4][2] = {};
   const int nk = (K + SG_K - 1) / SG_K;
 #pragma unroll
   for (int st = 0; st < SG_STAGES - 1; ++st) {
@@ -199,39 +241,20 @@ __global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
     const int nx = c + SG_STAGES - 1;
     if (nx < nk) load(nx % SG_STAGES, nx * SG_K);
     cp_async_commit();
-    const double* wp = wsm + (c % SG_STAGES) * SG_K * LDW + wm * 32 + 2 * gm;
-    const double* dp = dsm + (c % SG_STAGES) * SG_K * LDD + wn * 32 + 2 * gn;
-#pragma unroll 4
-    for (int kk = 0; kk < SG_K; ++kk) {
-      double2 w[4], d[2];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        w[i] = *reinterpret_cast<const double2*>(wp + kk * LDW + 8 * i);
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        d[j] = *reinterpret_cast<const double2*>(dp + kk * LDD + 16 * j);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          acc[2 * i][2 * j] = fma(w[i].x, d[j].x, acc[2 * i][2 * j]);
-          acc[2 * i][2 * j + 1] = fma(w[i].x, d[j].y, acc[2 * i][2 * j + 1]);
-          acc[2 * i + 1][2 * j] = fma(w[i].y, d[j].x, acc[2 * i + 1][2 * j]);
-          acc[2 * i + 1][2 * j + 1] = fma(w[i].y, d[j].y, acc[2 * i + 1][2 * j + 1]);
-        }
-    }
+    mma_chunk<LDW>(wsm + (c % SG_STAGES) * SG_K * LDW + wm * 32,
+                   dsm + (c % SG_STAGES) * SG_K * LDD + wn * 32, 1, LDD, acc, lane);
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const long long n = n0 + wn * 32 + 16 * j + 2 * gn;
+  for (int j = 0; j < 4; ++j) {
+    const long long n = n0 + wn * 32 + 8 * j + 2 * (lane & 3);
     if (n >= ntot) continue;
     double* out = dst + (n / nper) * nstride + n % nper;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int a = a0 + wm * 32 + 8 * (i >> 1) + 2 * gm + (i & 1);
+    for (int i = 0; i < 4; ++i) {
+      const int a = a0 + wm * 32 + 8 * i + (lane >> 2);
       if (a < K)
         *reinterpret_cast<double2*>(out + (chain_first(par) + 2ll * a) * rs) =
-            make_double2(acc[i][2 * j], acc[i][2 * j + 1]);
+            make_double2(acc[i][j][0], acc[i][j][1]);
     }
   }
 }
@@ -242,20 +265,21 @@ __global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
 // (x, y).  With `scale` the results are divided by the eigenvalue sums (zero
 // on the null modes), which ends the forward transforms.
 template <int WM>
-__global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
+__global__ void __launch_bounds__(64 * WM, SG_BLOCKS(WM))
     spec_lines(AxisBasis ax, int inverse, const double* __restrict__ src,
                double* __restrict__ dst, Geom g, int scale, const double* __restrict__ lx,
                const double* __restrict__ ly, double lam_floor) {
-  constexpr int THREADS = 64 * WM, LDW = 32 * WM, LDD = 2 * SG_K + 2, LDE = 64 * WM + 1;
+  constexpr int THREADS = 64 * WM, LDW = 32 * WM + SG_PAD, LDD = 2 * SG_K + 2;
+  constexpr int LDE = 64 * WM + 1;
   extern __shared__ __align__(16) double smem[];
-  double* wsm = smem;                                // [stage][chain][16][32 WM]
+  double* wsm = smem;                                // [stage][chain][16][32 WM + 8]
   double* dsm = smem + SG_STAGES * 2 * SG_K * LDW;   // [stage][32 lines][34]
   __shared__ long long loff[32];
   __shared__ double lsum[32];
-  const int a0 = blockIdx.y * LDW;
+  const int a0 = blockIdx.y * 32 * WM;
   const long long l0 = blockIdx.x * 32ll, nl = (long long)(g.nx - 2) * (g.ny - 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int par = warp / WM, wm = warp % WM, gm = lane >> 3, gn = lane & 7;
+  const int par = warp / WM, wm = warp % WM;
   if (tid < 32) {
     const long long l = l0 + tid;
     const int x = (int)(l / (g.ny - 2)) + 1, y = (int)(l % (g.ny - 2)) + 1;
@@ -267,7 +291,7 @@ __global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
   auto load = [&](int st, int c) {
 #pragma unroll
     for (int p = 0; p < 2; ++p)  // z = 32 c + 2 t: even chain position 16 c + t - 1
-      load_w<WM, THREADS>(wsm + (st * 2 + p) * SG_K * LDW, ax.W[inverse][p], ax.K[p],
+      load_w<WM>(wsm + (st * 2 + p) * SG_K * LDW, ax.W[inverse][p], ax.K[p],
                           c * SG_K - (p == 0 ? 1 : 0), a0, tid);
     const int z = 2 * SG_K * c + 2 * (tid & 15);
     for (int l = tid >> 4; l < 32; l += THREADS / 16) {
@@ -275,7 +299,7 @@ __global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
       cp_async16(dsm + (st * 32 + l) * LDD + 2 * (tid & 15), ok ? src + loff[l] + z : src, ok);
     }
   };
-  double acc[8][4] = {};
+  double acc[4][4][2] = {};
   const int nk = (g.nz - 1 + 2 * SG_K - 1) / (2 * SG_K);  // z = 0 .. nz-2
 #pragma unroll
   for (int st = 0; st < SG_STAGES - 1; ++st) {
@@ -288,37 +312,22 @@ __global__ void __launch_bounds__(64 * WM, WM >= 3 ? 2 : 4)
     const int nx = c + SG_STAGES - 1;
     if (nx < nk) load(nx % SG_STAGES, nx);
     cp_async_commit();
-    const double* wp = wsm + ((c % SG_STAGES) * 2 + par) * SG_K * LDW + wm * 32 + 2 * gm;
-    const double* dp = dsm + ((c % SG_STAGES) * 32 + gn) * LDD + (par == 0 ? 0 : 1);
-#pragma unroll 4
-    for (int kk = 0; kk < SG_K; ++kk) {
-      double2 w[4];
-      double d[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        w[i] = *reinterpret_cast<const double2*>(wp + kk * LDW + 8 * i);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) d[j] = dp[8 * j * LDD + 2 * kk];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[2 * i][j] = fma(w[i].x, d[j], acc[2 * i][j]);
-          acc[2 * i + 1][j] = fma(w[i].y, d[j], acc[2 * i + 1][j]);
-        }
-    }
+    mma_chunk<LDW>(wsm + ((c % SG_STAGES) * 2 + par) * SG_K * LDW + wm * 32,
+                   dsm + (c % SG_STAGES) * 32 * LDD + (par == 0 ? 0 : 1), LDD, 2, acc, lane);
   }
   cp_async_wait<0>();
   __syncthreads();  // the ring is free: rows of results take its place
   // odd chain's mode a at z = 1 + 2 a, even chain's at 2 + 2 a
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
-      smem[(gn + 8 * j) * LDE + 2 * (wm * 32 + 8 * (i >> 1) + 2 * gm + (i & 1)) +
-           (par == 0 ? 1 : 0)] = acc[i][j];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        smem[(8 * j + 2 * (lane & 3) + u) * LDE + 2 * (wm * 32 + 8 * i + (lane >> 2)) +
+             (par == 0 ? 1 : 0)] = acc[i][j][u];
   __syncthreads();
-  const int z0 = 1 + 2 * a0, zn = min(2 * LDW, g.nz - 2 + 1 - z0);
+  const int z0 = 1 + 2 * a0, zn = min(64 * WM, g.nz - 2 + 1 - z0);
   for (int l = warp; l < 32; l += THREADS / 32) {
     if (loff[l] < 0) continue;
     for (int r = lane; r < zn; r += 32) {
@@ -344,10 +353,10 @@ static int mode_units(int K) {
 }
 
 constexpr size_t spec_rows_smem(int wm) {
-  return sizeof(double) * SG_STAGES * SG_K * (32 * wm + 64);
+  return sizeof(double) * SG_STAGES * SG_K * (32 * wm + SG_PAD + 64 + SG_PAD);
 }
 constexpr size_t spec_lines_smem(int wm) {
-  const size_t ring = sizeof(double) * SG_STAGES * (2 * SG_K * 32 * wm + 32 * (2 * SG_K + 2));
+  const size_t ring = sizeof(double) * SG_STAGES * (2 * SG_K * (32 * wm + SG_PAD) + 32 * (2 * SG_K + 2));
   const size_t rows = sizeof(double) * 32 * (64 * wm + 1);
   return ring > rows ? ring : rows;
 }
@@ -430,23 +439,35 @@ __global__ void __launch_bounds__(TILE_THREADS)
              double* __restrict__ maxdiv) {
   __shared__ double red[32];
   double mx = 0.0;
-  auto ld = [&](const T* f, int x, int y, int z) -> double {
-    if (f == nullptr || !interior(g, x, y, z)) return 0.0;
-    return (double)f[(long long)x * s.sx + (long long)y * s.sy + (long long)z * s.sz];
-  };
   const int z = blockIdx.x * TILE_Z + threadIdx.x, y = blockIdx.y * TILE_Y + threadIdx.y;
   const int x0 = blockIdx.z * kSpecPlanes, x1 = min(x0 + kSpecPlanes, g.nx);
   if (z < g.pz && y < g.ny) {
-    for (int x = x0; x < x1; ++x) {
-      double div = 0.0;
-      if (interior(g, x, y, z)) {
-        const double tx = (ld(fx, x + 1, y, z) - ld(fx, x - 1, y, z)) * c2x;
-        const double ty = (ld(fy, x, y + 1, z) - ld(fy, x, y - 1, z)) * c2y;
-        const double tz = (ld(fz, x, y, z + 1) - ld(fz, x, y, z - 1)) * c2z;
-        div = (tx + ty) + tz;
-        mx = fmax(mx, fabs(div));
+    double* out = rhs + (long long)x0 * g.sxy + (long long)y * g.pz + z;
+    if (y >= 1 && y <= g.ny - 2 && z >= 1 && z <= g.nz - 2) {
+      // masked neighbours: those on the shell count as 0
+      const bool yp = y + 1 <= g.ny - 2, ym = y - 1 >= 1, zp = z + 1 <= g.nz - 2, zm = z - 1 >= 1;
+      const long long f0 = (long long)y * s.sy + (long long)z * s.sz;
+      auto at = [&](const T* f, int x, long long off, bool in) -> double {
+        return f != nullptr && in ? (double)f[(long long)x * s.sx + f0 + off] : 0.0;
+      };
+      auto fx_at = [&](int x) -> double { return at(fx, x, 0, x >= 1 && x <= g.nx - 2); };
+      double xm = fx_at(x0 - 1), xc = fx_at(x0);
+      for (int x = x0; x < x1; ++x, out += g.sxy) {
+        const double xp = fx_at(x + 1);
+        double div = 0.0;
+        if (x >= 1 && x <= g.nx - 2) {
+          const double tx = (xp - xm) * c2x;
+          const double ty = (at(fy, x, s.sy, yp) - at(fy, x, -s.sy, ym)) * c2y;
+          const double tz = (at(fz, x, s.sz, zp) - at(fz, x, -s.sz, zm)) * c2z;
+          div = (tx + ty) + tz;
+          mx = fmax(mx, fabs(div));
+        }
+        *out = -div;
+        xm = xc;
+        xc = xp;
       }
-      rhs[(long long)x * g.sxy + (long long)y * g.pz + z] = -div;
+    } else {
+      for (int x = x0; x < x1; ++x, out += g.sxy) *out = 0.0;
     }
   }
   // block max, then one atomic per block that raises it, on the bit pattern

@@ -371,24 +371,32 @@ __global__ void finish_kernel(StepArgs a, int done, void* uo, void* vo) {
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0 && a.flags) atomicOr(a.flags, 1);
 }
 
+constexpr int kConvertPlanes = 4;
 // dst = src * scale / rho  (see sw_convert)
 template <typename Tout, typename Trho>
 __global__ void convert_kernel(int ncomp, const double* __restrict__ src, Geom g, Tout* dst,
                                long long cs, long long sx, long long sy, long long sz,
                                double scale, const Trho* __restrict__ rho, long long rx,
                                long long ry, long long rz) {
-  const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n;
-       q += (long long)gridDim.x * blockDim.x) {
-    const int z = (int)(q % g.nz);
-    const long long xy = q / g.nz;
-    const int y = (int)(xy % g.ny);
-    const int x = (int)(xy / g.ny);
-    const long long i = xy * g.pz + z;
-    double f = scale;
-    if (rho) f = scale / (double)rho[x * rx + y * ry + z * rz];
-    for (int c = 0; c < ncomp; ++c)
-      dst[c * cs + x * sx + y * sy + z * sz] = (Tout)(src[c * g.ncell + i] * f);
+  // blocks of 32 (z) x 8 (y) threads, planes across the grid's z: no division
+  const int z = blockIdx.x * TILE_Z + threadIdx.x, y = blockIdx.y * TILE_Y + threadIdx.y;
+  if (z >= g.nz || y >= g.ny) return;
+  // four planes' loads in flight per component
+  const int x0 = blockIdx.z * kConvertPlanes, x1 = min(x0 + kConvertPlanes, g.nx);
+  const double* in = src + (long long)y * g.pz + z;
+  Tout* out = dst + y * sy + z * sz;
+  for (int c = 0; c < ncomp; ++c, in += g.ncell, out += cs) {
+    double v[kConvertPlanes];
+#pragma unroll
+    for (int k = 0; k < kConvertPlanes; ++k)
+      if (x0 + k < x1) v[k] = in[(x0 + k) * g.sxy];
+#pragma unroll
+    for (int k = 0; k < kConvertPlanes; ++k)
+      if (x0 + k < x1) {
+        double f = scale;
+        if (rho) f = scale / (double)rho[(x0 + k) * rx + y * ry + z * rz];
+        out[(x0 + k) * sx] = (Tout)(v[k] * f);
+      }
   }
 }
 
@@ -595,11 +603,12 @@ extern "C" int sw_convert(int ncomp, const double* src, int nx, int ny, int nz, 
     return SW_EINVAL;
   }
   Geom g = make_geom(nx, ny, nz, pad_pitch(nz));
-  const long long n = (long long)nx * ny * nz;
-  const int grid = grid_blocks(n, 256, 148 * 32);
+  const dim3 grid((unsigned)((nz + TILE_Z - 1) / TILE_Z), (unsigned)((ny + TILE_Y - 1) / TILE_Y),
+                  (unsigned)((nx + kConvertPlanes - 1) / kConvertPlanes));
+  const dim3 block(TILE_Z, TILE_Y);
   cudaStream_t s = (cudaStream_t)stream;
 #define SW_CONV(TO, TR)                                                                     \
-  convert_kernel<TO, TR><<<grid, 256, 0, s>>>(ncomp, src, g, (TO*)dst, dst_cs, dst_sx, dst_sy, \
+  convert_kernel<TO, TR><<<grid, block, 0, s>>>(ncomp, src, g, (TO*)dst, dst_cs, dst_sx, dst_sy, \
                                               dst_sz, scale, (const TR*)rho, rho_sx, rho_sy,  \
                                               rho_sz)
   if (out_dtype == SW_F32 && rho_dtype == SW_F32) SW_CONV(float, float);
