@@ -392,10 +392,10 @@ class _Run:
         # launch-wide tile queue of this solve's step launches
         self.queue = torch.zeros(2, dtype=torch.int32, device=dev)
         # force patterns and term table (set by set_patterns)
-        self.patterns = torch.zeros((1, 3, 0), dtype=self.dt, device=dev)
-        self.term_off = torch.zeros(self.n_steps + 1, dtype=torch.int32, device=dev)
-        self.term_pat = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.term_scale = torch.zeros(1, dtype=torch.float64, device=dev)
+        self.patterns = torch.empty((1, 3, 0), dtype=self.dt, device=dev)
+        none = torch.zeros(self.n_steps + 2, dtype=torch.int32, device=dev)
+        self.term_off, self.term_pat = none[:self.n_steps + 1], none[:1]
+        self.term_scale = none[:2].view(torch.float64)
         self.snaps = None
         self.trace_cells = None
         self.traces = None
@@ -435,11 +435,17 @@ class _Run:
 
     def set_patterns(self, pats: torch.Tensor, term_off, term_pat, term_scale):
         self.patterns = pats
-        self.term_off = torch.as_tensor(np.asarray(term_off, np.int32), device=self.dev)
-        if len(term_pat):
-            self.term_pat = torch.as_tensor(np.asarray(term_pat, np.int32), device=self.dev)
-            self.term_scale = torch.as_tensor(np.asarray(term_scale, np.float64),
-                                              device=self.dev)
+        # the three arrays in one copy: scales, then offsets, then patterns
+        n, m = max(1, len(term_pat)), len(term_off)
+        table = np.zeros(8 * n + 4 * (m + n), np.uint8)
+        ends = (8 * n, 8 * n + 4 * m, table.size)
+        table[:8 * len(term_pat)].view(np.float64)[:] = term_scale
+        table[ends[0]:ends[1]].view(np.int32)[:] = term_off
+        table[ends[1]:ends[1] + 4 * len(term_pat)].view(np.int32)[:] = term_pat
+        t = torch.from_numpy(table).to(self.dev)
+        self.term_scale = t[:ends[0]].view(torch.float64)
+        self.term_off = t[ends[0]:ends[1]].view(torch.int32)
+        self.term_pat = t[ends[1]:].view(torch.int32)
 
     def pattern_from_tensor(self, fs: torch.Tensor, dst: torch.Tensor, spacing_dt2: float):
         """Store a projected force (3 padded FP64 components) as a pattern of this form."""
@@ -639,23 +645,27 @@ class _Solve:
         self.run.pattern_from_tensor(fs_out, self.pats[k], self.dT * self.dT)
 
     def build_terms(self):
+        # one row per pattern slot: its scale at every step (a 4-D force's
+        # slices share the last row, at scale 1)
         f = self.forces
+        rows = [np.asarray(env, np.float64) for _c, env in f.separable]
+        if f.stream4d is not None:
+            rows.append((~f.zero_steps).astype(np.float64))
+        scale = np.stack(rows, axis=1) if rows else np.zeros((self.n_steps, 0))
+        used = scale != 0.0
+        step, slot = np.nonzero(used)  # in step order, then slot order
+        term_pat = slot.astype(np.int32)
         if self.stream_steps is not None:
-            self._stream_index = {it: j for j, it in enumerate(self.stream_steps)}
-        term_off, term_pat, term_scale = [0], [], []
-        for it in range(self.n_steps):
-            for k, (_c, env) in enumerate(f.separable):
-                s = float(env[it])
-                if s != 0.0:
-                    term_pat.append(k)
-                    term_scale.append(s)
-            if f.stream4d is not None and not f.zero_steps[it]:
-                term_pat.append(self.n_sep + (self._stream_index[it] if self.stream_steps
-                                              is not None else 0))
-                term_scale.append(1.0)
-            term_off.append(len(term_pat))
+            index = np.zeros(self.n_steps, np.int32)
+            index[self.stream_steps] = np.arange(len(self.stream_steps), dtype=np.int32)
+            last = slot == self.n_sep
+            term_pat[last] = self.n_sep + index[step[last]]
+        term_scale = scale[used]
+        count = used.sum(axis=1)
+        term_off = np.zeros(self.n_steps + 1, np.int32)
+        np.cumsum(count, out=term_off[1:])
         self.term_off = term_off
-        if max((b - a for a, b in zip(term_off, term_off[1:])), default=0) > _TWO_STEP_TERM_CAP:
+        if count.size and int(count.max()) > _TWO_STEP_TERM_CAP:
             # the two-steps-per-pass kernel holds at most this many force terms
             # of one step; more run one step per launch
             self.run.steps_per_pass = 1
