@@ -21,18 +21,24 @@
 // plane q and level 2 plane q-1.  Fifteen consumer warps each own one
 // level-1 row of 32 z pairs (packed .f32x2 arithmetic) and the same pairs at
 // level 2.  A thread walks its own column in registers at both levels (level
-// 0 of planes q-1 and q, level 1 of planes q-2, q-1 and q, the coefficients
-// of q-1) and takes the z neighbours from the lanes either side, so shared
-// memory serves only the rows either side, the column's next level-0 plane
-// and the coefficients: 30 eight-byte loads per pair and plane instead of
-// the 76 of reading every stencil point (shared-memory wavefronts 15.4 M
-// instead of 26 M in a launch at 192^3).
+// 0 of planes q-1 and q, level 1 of planes q-1 and q, the coefficients of
+// q-1) and takes the z neighbours from the lanes either side, so shared
+// memory serves only the rows either side, the column's next level-0 plane,
+// its level 1 of plane q-2 and the coefficients: 36 eight-byte loads per pair
+// and plane instead of the 76 of reading every stencil point.  Plane q-2 comes
+// from the ring, where the thread itself wrote it, because with it in
+// registers too the loop cannot be unrolled by two without spilling, and
+// unrolled the planes of a column change names instead of registers (52 moves
+// of 377 instructions a plane): 600 steps with a push's projection at 256 x
+// 256 x 384 145.5 -> 139.5 ms, 500 steps at 64^3 3.65 -> 3.54 ms; 1000 steps
+// at 192^3, where the power limit holds the clock, 54.7 -> 54.0 ms.
 //
 // Two waits per plane and warp.  The level-1 ring has one mbarrier per slot
 // (one arrival per warp, when its row of the plane is written); level 2 of
 // plane q-1 waits for that plane.  Four slots need no barrier for their
 // reuse: a warp that has seen plane q-2 complete knows that every warp has
-// left iteration q-3, the last to read the slot plane q goes to.  With a
+// left iteration q-3, the last to read the slot plane q goes to (a thread's
+// own element of it is read once more, by that thread, in iteration q-2).  With a
 // barrier of its own for the coefficients and one for the reuse of a slot
 // (four waits per plane) a quarter of the kernel's instructions were waits.
 // Columns in registers and two waits: 104 instead of 115 us per launch at
@@ -252,11 +258,11 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
   const int slot1 = snap1 ? (lit + 1) / in->snap_stride - 1 : 0;
   const int slot2 = snap2 ? (lit + 2) / in->snap_stride - 1 : 0;
   // Each thread walks its own column in registers: level 0 of planes q-1 and
-  // q, level 1 of planes q-2 and q-1 (u and d of three components).  Shared
-  // memory is read only for what other threads hold: the rows either side at
-  // both levels, and the column's next level-0 plane.
+  // q, level 1 of plane q-1 (u and d of three components).  Shared memory is
+  // read for what other threads hold (the rows either side at both levels),
+  // the column's next level-0 plane and its level 1 of plane q-2.
   float2 au[3], ad[3], bu[3], bd[3];  // level 0: planes q-1, q
-  float2 eu[3], ed[3], fu[3], fd[3];  // level 1: planes q-2, q-1
+  float2 fu[3], fd[3];                // level 1: plane q-1
   const float2 zero2 = make_float2(0.f, 0.f);
   float2 Mp = zero2, Ep = zero2;  // coefficients of the previous plane
   {
@@ -265,7 +271,7 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
     for (int c = 0; c < 3; ++c) {
       au[c] = tb_ld2(P0 + c * H * W);
       ad[c] = VISC ? tb_ld2(P0 + (3 + c) * H * W) : zero2;
-      eu[c] = ed[c] = fu[c] = fd[c] = zero2;
+      fu[c] = fd[c] = zero2;
     }
   }
   __syncwarp();
@@ -285,6 +291,7 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
       bd[c] = tb_ld2(P0 + (3 + c) * H * W);
     }
   }
+#pragma unroll 2
   for (int q = tc.x0 - 1; q <= tc.x1; ++q) {
     const RingPos<T::NA> nxt = p.ca;  // plane q+1
     if (!ws_wait(&k.hd->fullA[nxt.s], nxt.ph, k.abort_flag)) {
@@ -366,6 +373,7 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
     if (q > tc.x0 && warp_out) {
       // ---- level 2: step lit+2 at plane x = q-1 on the output tile ----
       const float* Lc = k.ringL + p.lp.s * LF + ol2;  // a row of the output tile
+      const float* Le = k.ringL + ((p.lp.s + T::NL - 1) & (T::NL - 1)) * LF + ol;  // plane q-2
       const int x = q - 1;
       const long long i = (long long)x * g.sxy + (long long)y * g.pz + zp;
       float* sp = nullptr;
@@ -377,7 +385,8 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
         const float* Pc = Lc + c * LP;
         const float* Pd = Lc + (3 + c) * LP;
         const float2 inc = tb_inc<VISC, DAMP, PUSH>(
-            fu[c], fd[c], nu[c], nd[c], eu[c], ed[c], tb_ld2(Pc + LZ), tb_ld2(Pc - LZ),
+            fu[c], fd[c], nu[c], nd[c], tb_ld2(Le + c * LP),
+            VISC ? tb_ld2(Le + (3 + c) * LP) : zero2, tb_ld2(Pc + LZ), tb_ld2(Pc - LZ),
             VISC ? tb_ld2(Pd + LZ) : zero2, VISC ? tb_ld2(Pd - LZ) : zero2, Mp, Ep, lk, damp,
             tbuf.t[1], PUSH && store ? n2 : 0, c * (long long)nc + i, 0);
         const float2 un = fadd2(fu[c], inc);
@@ -393,9 +402,7 @@ __device__ __forceinline__ TbPos tb_tile(const TmaF32TB* __restrict__ in, int lo
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      eu[c] = fu[c];
       fu[c] = nu[c];
-      if (VISC) ed[c] = fd[c];
       fd[c] = nd[c];
     }
     Mp = Mc;
@@ -426,7 +433,7 @@ __device__ __forceinline__ bool tb_snaps(const TmaF32TB* __restrict__ in, int li
 // calls (~3 local loads per warp and plane), and with the force terms read
 // from the solve's tables inside the loop the push loop spilled (push tiles
 // 4.9x slower).  With the terms in the shared term buffer the whole kernel
-// fits 128 registers with nothing spilled.  (Running the push and snapshot
+// fits 128 registers with one to three of them spilled.  (Running the push and snapshot
 // tiles in a second launch of their own, which kept the first launch's
 // variant at 102 registers, measured 1.4 % slower than this one launch.)
 template <int LZ, bool VISC, bool DAMP>
