@@ -18,6 +18,7 @@
 //      vector:  b_i = (2 alpha_Np / c) mean(p v_i)
 // Both passes are HBM-bound reads of the pressure (and velocity) records.
 #include <algorithm>
+#include <type_traits>
 
 #include "sw_common.cuh"
 
@@ -133,16 +134,23 @@ struct ArfGate {
 // One lane's sums over its windows of a row: every G-th 16-byte window from
 // `sub` on, `nw` in all, the row's first window at element e0 of the records,
 // the gate's first sample n0 elements after it; the gate's bits tell which of a
-// window's elements count.  Two windows of one record, or one of four, are in
-// flight per lane: more take registers from the warps that hide the latency
-// (four of four: 120 registers, 16 warps per SM, 15 % slower).
+// window's elements count.  Four windows of one record, or one of four, are in
+// flight per lane: with two of one record the reads did not fill DRAM (405 of
+// 1349 samples on 90 x 96 x 100 cells 298 us, with four 248, with eight 250 and
+// small grids slower), and with four records more windows take registers from
+// the warps that hide the latency (four: 120 registers, 16 warps per SM, 15 %
+// slower; two at 80 registers: no faster on large grids).
 template <typename T, int NF, int G>
 __device__ __forceinline__ void row_sums(const T* __restrict__ p, const T* __restrict__ q0,
                                          const T* __restrict__ q1, const T* __restrict__ q2,
                                          long long e0, int sub, int nw, int n0,
                                          const unsigned* bits, double (&s)[3]) {
   constexpr int V = ArfWin<T>::V;
-  constexpr int B = NF == 1 ? 2 : 1;
+  constexpr int B = NF == 1 ? 4 : 1;
+  // four chains for the one sum, so that few lanes a cell round no more than
+  // many would; one for each of three (two spill, and are 2 % slower)
+  constexpr int C = NF == 1 ? 4 : 1, S = NF == 1 ? 1 : 3;
+  double acc[S][C] = {};
   e0 += sub * V;
   for (int w0 = sub; w0 < nw; w0 += B * G, e0 += B * G * V) {
     ArfWin<T> a[B], b[B], c[B], d[B];
@@ -165,15 +173,24 @@ __device__ __forceinline__ void row_sums(const T* __restrict__ p, const T* __res
       for (int u = 0; u < V; ++u) {
         if (((in >> u) & 1u) == 0u) continue;
         const double pv = (double)a[k].v[u];
+        const int n = (k * V + u) & (C - 1);
         if (NF == 1) {
-          s[0] = fma(pv, pv, s[0]);
+          acc[0][n] = fma(pv, pv, acc[0][n]);
         } else {
-          s[0] = fma(pv, (double)b[k].v[u], s[0]);
-          s[1] = fma(pv, (double)c[k].v[u], s[1]);
-          s[2] = fma(pv, (double)d[k].v[u], s[2]);
+          acc[0][n] = fma(pv, (double)b[k].v[u], acc[0][n]);
+          acc[1 % S][n] = fma(pv, (double)c[k].v[u], acc[1 % S][n]);
+          acc[2 % S][n] = fma(pv, (double)d[k].v[u], acc[2 % S][n]);
         }
       }
     }
+  }
+#pragma unroll
+  for (int f = 0; f < S; ++f) {
+#pragma unroll
+    for (int n = C / 2; n > 0; n /= 2)
+#pragma unroll
+      for (int u = 0; u < n; ++u) acc[f][u] += acc[f][u + n];
+    s[f] = acc[f][0];
   }
 }
 
@@ -190,8 +207,8 @@ __device__ __forceinline__ void row_sums(const T* __restrict__ p, const T* __res
 // sum, then evaluates the formula for all of them at once: its float64
 // divisions in one lane per group took as long as the reads.  Measured against
 // one gate entry at a time and one cell per warp: 109 of 300 samples of a float
-// record on 128 x 96 x 112 cells 363 -> 167 us, 129 of 257 of four records on
-// 80 x 72 x 101 cells 382 -> 252 us (6 TB/s of DRAM reads, whose granules are
+// record on 128 x 96 x 112 cells 363 -> 134 us, 129 of 257 of four records on
+// 80 x 72 x 101 cells 382 -> 242 us (6 TB/s of DRAM reads, whose granules are
 // wider than the gate).
 template <typename T, typename To, int NF, int G>
 __global__ void __launch_bounds__(256, 4)
@@ -314,30 +331,38 @@ int launch_force(const void* p, const void* const* q, long long ncell, int nt, c
       (NF == 1 || (((uintptr_t)q[0] & 15u) == al && ((uintptr_t)q[1] & 15u) == al &&
                    ((uintptr_t)q[2] & 15u) == al));
   // lanes per cell: as few as keep a gate to several loads per lane (the
-  // group's reduction costs log2 G shuffles a cell), a warp for long gates
-  // (their rows are whole DRAM bursts already)
-  // rounds of 32 / g cells per warp: up to the 32 cells whose formula one warp
-  // evaluates at once, fewer where the grid would not fill the GPU
+  // group's reduction costs log2 G shuffles a cell).  With four records a lane
+  // has a quarter of the windows of one record in flight, and longer runs of
+  // one row make up for it.  On 29 x 116 x 74 cells, us at 8, 16 and 32 lanes:
+  // one record, 109 / 405 / 1200 samples: 31 40 61 / 83 84 90 / 208 206 217;
+  // four records, 72 / 109 / 200 / 600 samples: 77 79 89 / 101 97 100 /
+  // 165 157 160 / 443 410 392.
+  // Rounds of 32 / g cells per warp: up to the 32 cells whose formula one warp
+  // evaluates at once, fewer where the grid would not fill the 32 warps an SM
+  // holds (four records, 405 samples on 34 x 33 x 23 cells: 41 us with half of
+  // them, 35 us so).
   int iters = 1;
   auto blocks = [&](int g) {
-    const long long warps = 16LL * kNumSMs, rounds = (ncell * g + 31) / 32;
-    iters = (int)std::max<long long>(1, std::min<long long>(g, rounds / warps));
+    const long long warps = 32LL * kNumSMs, rounds = (ncell * g + 31) / 32;
+    iters = (int)std::max<long long>(1, std::min<long long>(g, (rounds + warps - 1) / warps));
     const long long want = (rounds + iters * 8 - 1) / (iters * 8);
     return (int)std::max<long long>(1, std::min<long long>(want, 16LL * kNumSMs));
   };
-  if (ngate <= 32) {
-    const int nb = blocks(4);
-    arf_force<T, To, NF, 4><<<nb, 256, 0, s>>>(pp, qa, qb, qc, ncell, nt, gate, ngate, m, f0_mhz,
+  auto launch = [&](auto lanes) {
+    constexpr int G = decltype(lanes)::value;
+    const int nb = blocks(G);
+    arf_force<T, To, NF, G><<<nb, 256, 0, s>>>(pp, qa, qb, qc, ncell, nt, gate, ngate, m, f0_mhz,
                                                oa, ob, oc, windows, iters);
-  } else if (ngate <= 512) {
-    const int nb = blocks(8);
-    arf_force<T, To, NF, 8><<<nb, 256, 0, s>>>(pp, qa, qb, qc, ncell, nt, gate, ngate, m, f0_mhz,
-                                               oa, ob, oc, windows, iters);
-  } else {
-    const int nb = blocks(32);
-    arf_force<T, To, NF, 32><<<nb, 256, 0, s>>>(pp, qa, qb, qc, ncell, nt, gate, ngate, m, f0_mhz,
-                                                oa, ob, oc, windows, iters);
-  }
+  };
+  using std::integral_constant;
+  if (ngate <= 32)
+    launch(integral_constant<int, 4>());
+  else if (ngate <= (NF == 1 ? 1024 : 96))
+    launch(integral_constant<int, 8>());
+  else if (NF == 1 || ngate <= 256)
+    launch(integral_constant<int, 16>());
+  else if constexpr (NF == 3)
+    launch(integral_constant<int, 32>());
   count_launches(1);
   SW_CHECK_LAUNCH("radiation force");
   return SW_OK;

@@ -70,3 +70,25 @@ def test_envelope(cuda, ncell, nt, dtype):
     env = ops.arf_envelope(torch.as_tensor(p, device=cuda), ncell, nt).cpu().numpy()
     ref = (p.astype(np.float64) ** 2).mean(0)
     assert np.all(np.abs(env - ref) <= 1e-12 * ref)
+
+
+@pytest.mark.parametrize("gate", [slice(2, 30), slice(5, 85), slice(0, 100), slice(0, 109)])
+def test_several_rounds_per_warp(cuda, gate):
+    # enough cells that a warp takes more than one round of every lane split,
+    # the last one partly empty; at most 109 samples: the same bound
+    import torch
+
+    import shearwave_b200 as sw
+
+    shape, nt = (33, 41, 37), 109
+    rng = np.random.default_rng(gate.stop)
+    host = [rng.standard_normal((*shape, nt)) for _ in range(4)]
+    rec = [torch.as_tensor(h, device=cuda) for h in host]
+    idx = np.arange(nt)[gate]
+    out = sw.compute_radiation_force(rec[0], 1540.0, 1000.0, 0.5, 5e6, gate=gate)
+    ref, scale = _reference(host[0], host[0], 1540.0, 1000.0, 0.5, 5e6, idx)
+    assert np.all(np.abs(out.cpu().numpy() - ref) <= 1e-13 * scale)
+    outs = sw.compute_radiation_force_velocity(*rec, 1540.0, 1000.0, 0.5, 5e6, gate=gate)
+    for o, v in zip(outs, host[1:]):
+        ref, scale = _reference(host[0], v, 1540.0, 1000.0, 0.5, 5e6, idx)
+        assert np.all(np.abs(o.cpu().numpy() - ref) <= 1e-13 * scale)
