@@ -269,7 +269,10 @@ typedef struct sw_fdtd_desc {
   int32_t kernel;         /* 0: TMA-staged step kernels (default), 1: direct-load kernels */
   /* Device int the step loop may use as its step counter: with it, long runs
    * of sw_fdtd_steps replay one instantiated CUDA graph of 32 steps instead
-   * of launching every step (NULL: direct launches only). */
+   * of launching every step (NULL: direct launches only).  With `queue` as
+   * well, pairs of steps of the F32 form run in resident launches of up to
+   * 512 pairs each; their progress words lie in the x = 0 shell plane of
+   * component 6 of state[0], and are zero again when a call's work is done. */
   int32_t* clock;
   /* Two device int32s, zero at the first call (the kernels leave them zero):
    * the launch-wide tile queue of this solve's own step launches, which
