@@ -260,7 +260,8 @@ struct CgTile {
 // one ahead (unit u holds planes 2u and 2u + 1 of the walk); in the update
 // phase the point-wise planes of a unit, on the barrier of the unit ahead.
 // (Their ring needs no barrier for its reuse: a free stage means that the unit
-// CR_NA - 1 = CR_NB before the point-wise one being loaded is done.)  Of a
+// CR_NA - 1 = CR_NB before the point-wise one being loaded is done, its points
+// included: consumers release a unit's stage after they have read both.)  Of a
 // last unit with one plane of the tile the other plane is loaded too and never
 // used.  The tile's number goes with its first unit.
 template <bool UPDATE>
@@ -439,11 +440,11 @@ __device__ __forceinline__ bool ring_tile(const CgInst& in, const TileCoord& tc,
       ap1 = stencil1(A + I1, c1, c0, f0, two ? i + step : i);
       bk = c1;
     }
-    release(s0);
     const double* B = q.points();
     finish(c0, ap0, B + B0, i, aa, ab);
     finish(c1, ap1, B + B1, i + step, aa && two, ab && two);
     if (UPDATE) q.next_points();
+    release(s0);  // after the unit's points too: their room is reused on its word
     c0 = f0;
     c1 = f1;
     s0 = s1;
