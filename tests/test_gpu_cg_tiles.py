@@ -76,3 +76,19 @@ def test_batched_projection_with_ended_and_tiny_instances(cuda):
         both = outs[k].reshape(3, s[0], s[1], pz)[..., :s[2]]
         assert all(torch.equal(a, b) for a, b in zip(alone, both)), k
         assert int(stats[k, 0]) == info["iters"]
+
+
+@pytest.mark.parametrize("shape", [(69, 113, 147), (118, 105, 79)])
+def test_repeats_are_bitwise(cuda, shape):
+    # every sum is in a fixed order, so any difference is a race in the rings
+    import torch
+
+    import shearwave_b200 as sw
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    f = [torch.randn(shape, device=cuda, dtype=torch.float64, generator=g) for _ in range(3)]
+    first = None
+    for _ in range(60):
+        out = sw.project_vector_field(*f, 5e-4, 5e-4, 5e-4, 1e-10, 300)
+        first = [o.clone() for o in out] if first is None else first
+        assert all(torch.equal(a, b) for a, b in zip(out, first))
