@@ -500,7 +500,12 @@ __device__ __forceinline__ bool tb_wait_around(const TmaF32TB& in, const TbProgr
   while (true) {
     int v = need;
     if (mine) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(w) : "memory");
-    if (__all_sync(0xffffffffu, v >= need)) return true;
+    if (__all_sync(0xffffffffu, v >= need)) {
+      // votes do not order memory: every lane's acquire before the copies that
+      // one lane issues for the warp
+      __syncwarp();
+      return true;
+    }
     const bool late = (((uint32_t)clock() - t0) >> 10) > (uint32_t)abort_flag[1];
     if (late) *abort_flag = 1;
     if (__any_sync(0xffffffffu, late || *abort_flag != 0 || solve_abandoned(in.flags)))

@@ -1,0 +1,36 @@
+"""Ordering rules of the kernels that no run can show (no GPU).
+
+A missing warp barrier or fence lets a lane run ahead once in many runs, if at
+all, so these rules are read off the sources: each test finds the place that
+has to be ordered and looks for what orders it.
+"""
+
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parents[1] / "shearwave_b200" / "csrc"
+
+
+def _source(name):
+    """A source file without comments, white space collapsed."""
+    text = (CSRC / name).read_text()
+    return re.sub(r"\s+", " ", re.sub(r"//[^\n]*", "", text))
+
+
+def _body(text, head):
+    """The braces that follow the first match of ``head``."""
+    start = text.index("{", re.search(head, text).end())
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError(head)
+
+
+def test_neighbours_progress_is_ordered_before_the_copies():
+    # 27 lanes acquire a neighbour's word each, one lane issues the copies;
+    # a vote between them orders no memory
+    body = _body(_source("sw_step_tb.cu"), r"bool tb_wait_around\([^{]*")
+    done = body.index("v >= need")
+    assert "__syncwarp()" in body[done:body.index("return true", done)]
