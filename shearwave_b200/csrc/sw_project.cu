@@ -730,6 +730,7 @@ __global__ void __launch_bounds__(CR_THREADS, 2)
           for (int u = (tc.x1 - tc.x0 + 1) / 2 + 2; u > 0 && ok; --u) {
             ok = ws_wait(&q.hd->full[q.a.s], q.a.ph, q.abort_flag);
             if (!ok) break;
+            __syncwarp();  // every lane has seen the stage's phase (and its tile)
             if (lane == 0) mbar_arrive(&q.hd->empty[q.a.s]);
             if (update && u <= (tc.x1 - tc.x0 + 1) / 2) q.next_points();
             q.a.next();

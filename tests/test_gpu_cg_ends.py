@@ -1,0 +1,31 @@
+"""The ends of CG solves: instances that end at different phases of a launch,
+and solves that break down, over and over."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_instances_that_end_one_after_another(cuda):
+    """A phase drains the tiles of an instance that ends at its start, beside the
+    tiles of others; each instance keeps the bits of its own run every time."""
+    import torch
+
+    import shearwave_b200 as sw
+    from shearwave_b200 import ops
+
+    # more tiles than blocks, both tile shapes, limits one update apart
+    shapes = [(40, 33, 70), (33, 34, 66), (21, 50, 33), (17, 19, 33)] * 5
+    iters = [1 + k % 7 for k in range(len(shapes))]
+    h = 0.5e-3
+    rng = np.random.default_rng(11)
+    f = [[torch.as_tensor(rng.standard_normal(s), device=cuda) for _ in range(3)] for s in shapes]
+    alone = [sw.project_vector_field(*c, h, h, h, 1e-12, n) for c, n in zip(f, iters)]
+    for _ in range(10):
+        outs, stats = ops.project_batch([c[0] for c in f], [c[1] for c in f], [c[2] for c in f],
+                                        [h] * 3 * len(f), [1e-12] * len(f), iters)
+        for k, s in enumerate(shapes):
+            both = outs[k].reshape(3, s[0], s[1], ops.pitch(s[2]))[..., :s[2]]
+            assert all(torch.equal(a, b) for a, b in zip(alone[k], both)), k
+            assert int(stats[k, 0]) == iters[k]

@@ -8,6 +8,8 @@ has to be ordered and looks for what orders it.
 import re
 from pathlib import Path
 
+import pytest
+
 CSRC = Path(__file__).resolve().parents[1] / "shearwave_b200" / "csrc"
 
 
@@ -34,3 +36,15 @@ def test_neighbours_progress_is_ordered_before_the_copies():
     body = _body(_source("sw_step_tb.cu"), r"bool tb_wait_around\([^{]*")
     done = body.index("v >= need")
     assert "__syncwarp()" in body[done:body.index("return true", done)]
+
+
+@pytest.mark.parametrize("name", ["sw_project.cu", "sw_step_tb.cu", "sw_step_tma.cu"])
+def test_a_warp_leaves_a_stage_together(name):
+    # lane 0 frees a ring stage for its warp: not while another lane still
+    # reads the stage, its slot or its barrier's phase
+    text = _source(name)
+    frees = [m.start() for m in re.finditer(r"mbar_arrive\(&[\w.>-]*empty", text)]
+    assert frees
+    for at in frees:
+        guard = text.rindex("if (lane == 0)", 0, at)
+        assert text[:guard].rstrip().endswith("__syncwarp();"), text[guard - 120:at + 40]
