@@ -458,9 +458,12 @@ __device__ __forceinline__ bool ring_tile(const CgInst& in, const TileCoord& tc,
 // launch): arrivals are counted in one word, the last one raises the other,
 // which the waiting blocks poll (on a line of its own, so the polls do not
 // hold up the arrivals).  Bounded; an error raised by any block, or a wait
-// that ran out in this one, ends it.
+// that ran out in this one, ends it.  Returns whether the block goes on: with
+// `run` (a single instance's, written by thread 0), only while *run holds.  It
+// is read here, by its writer, because no warp can read it after the barrier:
+// the consumers may be in the next phase by then and have changed it.
 __device__ __forceinline__ bool cg_grid_sync(CgGrid b, unsigned int n, volatile int* abort_flag,
-                                             int* ok_s) {
+                                             const int* run, int* ok_s) {
   asm volatile("fence.proxy.async;" ::: "memory");  // this phase's stores, next phase's TMA reads
   __syncthreads();
   if (*abort_flag) return false;  // the same in every thread: set before the barrier, if at all
@@ -489,7 +492,7 @@ __device__ __forceinline__ bool cg_grid_sync(CgGrid b, unsigned int n, volatile 
         }
       }
     }
-    *ok_s = ok;
+    *ok_s = ok && (run == nullptr || *run);
   }
   __syncthreads();
   asm volatile("fence.proxy.async;" ::: "memory");
@@ -758,8 +761,8 @@ __global__ void __launch_bounds__(CR_THREADS, 2)
     if (!coop) break;
     // a single instance ends in every block alike; the owner has recorded why
     // (a breakdown found in an update phase ends the next apply phase)
-    if (!cg_grid_sync(bar, ++nsync, q.abort_flag, &ok_s)) break;
-    if (ninst == 1 && !update && !cc.run) break;
+    const int* run = ninst == 1 && !update ? &cc.run : nullptr;
+    if (!cg_grid_sync(bar, ++nsync, q.abort_flag, run, &ok_s)) break;
   }
   __syncthreads();
   if (*q.abort_flag && warp == CR_WARPS && lane == 0) {

@@ -29,3 +29,20 @@ def test_instances_that_end_one_after_another(cuda):
             both = outs[k].reshape(3, s[0], s[1], ops.pitch(s[2]))[..., :s[2]]
             assert all(torch.equal(a, b) for a, b in zip(alone[k], both)), k
             assert int(stats[k, 0]) == iters[k]
+
+
+@pytest.mark.parametrize("shape", [(5, 6, 7), (17, 19, 33), (40, 33, 70)])
+def test_breakdowns_end_the_launch(cuda, shape):
+    """A negative modulus makes p.Ap negative: the first update phase finds it and the
+    next phase ends the launch, every time, without a wait that runs out."""
+    import torch
+
+    import shearwave_b200 as sw
+
+    g = torch.Generator(device="cuda").manual_seed(1)
+    b = torch.randn(shape, device=cuda, dtype=torch.float64, generator=g)
+    info = {}
+    for _ in range(300):
+        out = sw.elastic_solve_static(b, 0.5, 0.5, 0.5, -1.0, tol=1e-9, max_iters=50, info=info)
+        assert info["iters"] == 0
+    assert not bool(out.any())

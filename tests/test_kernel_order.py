@@ -48,3 +48,14 @@ def test_a_warp_leaves_a_stage_together(name):
     for at in frees:
         guard = text.rindex("if (lane == 0)", 0, at)
         assert text[:guard].rstrip().endswith("__syncwarp();"), text[guard - 120:at + 40]
+
+
+def test_a_block_decides_to_leave_before_its_barrier():
+    # the consumers may be in the next phase, and have changed cc.run, when the
+    # producer's warp comes out of the grid barrier
+    text = _source("sw_project.cu")
+    kernel = _body(text, r"cg_ring\(const CgInst")
+    after = kernel[kernel.index("cg_grid_sync("):]
+    assert "cc." not in after[after.index(";"):]
+    sync = _body(text, r"bool cg_grid_sync\([^{]*")
+    assert "*run" in sync[sync.index("if (threadIdx.x == 0)"):sync.rindex("__syncthreads()")]
