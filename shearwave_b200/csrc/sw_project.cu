@@ -664,8 +664,10 @@ __global__ void __launch_bounds__(CR_THREADS, 2)
             pt.t = t;
             pt.lz = rg->lz;
             pt.tc = tile_coord_t(in.g, rg->tr, t - in.ring_base, pt.lz, 512 / pt.lz);
-            for (const CUtensorMap* m : {&rg->ph[0], &rg->ph[1], &rg->rh, &rg->rp, &rg->xp})
+            for (const CUtensorMap* m : {&rg->ph[0], &rg->ph[1], &rg->rh, &rg->rp, &rg->xp}) {
+              tmap_acquire(m);
               prefetch_tmap(m);
+            }
           }
           // (a single instance runs until every block leaves)
           if ((ninst > 1 || !coop) && __ldcg(&pt.st->reason) != SW_CG_RUNNING) continue;

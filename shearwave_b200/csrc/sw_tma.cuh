@@ -88,6 +88,15 @@ __device__ inline void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* 
       : "memory");
 }
 
+// Before the first use, by this thread, of a tensor map in global memory (not of
+// one in a kernel's parameters): the map was written through another proxy than
+// the one that reads it, at an address that may have held another map before.
+__device__ inline void tmap_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(
+                   reinterpret_cast<uint64_t>(map))
+               : "memory");
+}
+
 __device__ inline void prefetch_tmap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }

@@ -46,3 +46,31 @@ def test_breakdowns_end_the_launch(cuda, shape):
         out = sw.elastic_solve_static(b, 0.5, 0.5, 0.5, -1.0, tol=1e-9, max_iters=50, info=info)
         assert info["iters"] == 0
     assert not bool(out.any())
+
+
+def test_grids_one_after_another_in_one_workspace(cuda):
+    """The tensor maps of a solve lie in its workspace: another grid's, at the same
+    address, are not used for it."""
+    import ctypes as C
+
+    import torch
+
+    import shearwave_b200 as sw
+    from shearwave_b200 import _native, ops
+
+    shapes = [(20, 30, 40), (30, 20, 40), (12, 50, 33), (40, 30, 20)]
+    h = 0.5e-3
+    g = torch.Generator(device="cuda").manual_seed(5)
+    f = [[torch.randn(s, device=cuda, dtype=torch.float64, generator=g) for _ in range(3)]
+         for s in shapes]
+    ref = [sw.project_vector_field(*c, h, h, h, 1e-9, 30) for c in f]
+    nb = max(int(_native.load().sw_project_workspace_bytes(*s)) for s in shapes)
+    ws = torch.empty(nb, dtype=torch.uint8, device=cuda)
+    for k in list(range(len(shapes))) * 25:
+        nx, ny, nz = shapes[k]
+        out = torch.empty((3, nx, ny, ops.pitch(nz)), dtype=torch.float64, device=cuda)
+        st = _native.CGStats()
+        _native.call("sw_project", _native.SW_F64, *(c.data_ptr() for c in f[k]), ny * nz, nz, 1,
+                     nx, ny, nz, h, h, h, 1e-9, 30, out.data_ptr(), ws.data_ptr(), nb,
+                     C.byref(st), torch.cuda.current_stream().cuda_stream)
+        assert all(torch.equal(a, b) for a, b in zip(out[..., :nz], ref[k])), k

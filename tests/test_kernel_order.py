@@ -59,3 +59,10 @@ def test_a_block_decides_to_leave_before_its_barrier():
     assert "cc." not in after[after.index(";"):]
     sync = _body(text, r"bool cg_grid_sync\([^{]*")
     assert "*run" in sync[sync.index("if (threadIdx.x == 0)"):sync.rindex("__syncthreads()")]
+
+
+def test_cg_acquires_its_tensor_maps():
+    # they lie in a workspace that may have held another grid's maps
+    kernel = _body(_source("sw_project.cu"), r"cg_ring\(const CgInst")
+    assert 0 <= kernel.find("tmap_acquire(m)") < kernel.index("prefetch_tmap(m)")
+    assert kernel.index("prefetch_tmap(m)") < kernel.index("ring_load<")
