@@ -575,6 +575,7 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
     RingPos<NA> pa;
     RingPos<NB> pb;
     bool ok = true;
+    int acquired = -1;  // the solve whose tensor maps are acquired
     // one lane: the planes of one tile (`tag` goes to the consumers with it)
     auto load_tile = [&](const T* in, int k, int tag, int t, int local, int lit, bool push) {
       const int ord = lg->n_taken;  // the tile's ordinal: its term buffer
@@ -584,6 +585,11 @@ __global__ void __launch_bounds__(TmaF32TB::THREADS, 1)
       const TbDims dm = LZ == 32 || (LZ == 0 && in->lz == 32) ? tb_dims<32>() : tb_dims<64>();
       const TbCoord tc = tb_coord_rt(g, in->ts, local, dm.oz, dm.oy);
       const CUtensorMap* tma = &in->tm[lit % 3];
+      if (BATCH && k != acquired) {
+        tmap_acquire(tma);
+        tmap_acquire(&in->tmm);
+        acquired = k;
+      }
       const uint32_t bbytes = dm.b_cells * 4 * in->ncoef;
       bool first = true;
       // level-0 plane p, and from plane x0 on the coefficients of plane p-1

@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(TmaF32::THREADS, TmaF32::MIN_CTAS)
     if (lane == 0) {
       RingPos<NA> pa;  // next stage of ring A / ring B to load
       RingPos<NB> pb;
-      int stride_next = blockIdx.x;
+      int stride_next = blockIdx.x, acquired = -1;  // the solve whose maps are acquired
       while (!*abort_flag) {
         const int t = next_tile(queue, stride_next);
         if (t >= ntiles) {  // end of this CTA's work: arm one stage without a copy
@@ -397,6 +397,12 @@ __global__ void __launch_bounds__(TmaF32::THREADS, TmaF32::MIN_CTAS)
         const CUtensorMap* tma = &in->tm[lit % 3];
         const CUtensorMap* tmc = &in->tmc[lit % 3];
         const bool kahan = KR && in->kahan;  // the compact ring never carries c
+        if (BATCH && k != acquired) {
+          tmap_acquire(tma);
+          if (kahan) tmap_acquire(tmc);
+          tmap_acquire(&in->tmm);
+          acquired = k;
+        }
         const uint32_t pbytes = (kahan ? TmaF32::C_BYTES : 0) + TZ * TY * 4 * in->ncoef;
         for (int p = tc.x0 - 1; p <= tc.x1 && !*abort_flag; ++p) {
           const int sa = pa.s;
@@ -502,7 +508,7 @@ __global__ void __launch_bounds__(TmaF64::THREADS, 2)
     if (lane == 0) {
       RingPos<NA> pa;
       RingPos<NB> pb;
-      int stride_next = blockIdx.x;
+      int stride_next = blockIdx.x, acquired = -1;  // the solve whose maps are acquired
       while (!*abort_flag) {
         const int t = next_tile(queue, stride_next);
         if (t >= ntiles) {  // end of this CTA's work: arm one stage without a copy
@@ -522,6 +528,12 @@ __global__ void __launch_bounds__(TmaF64::THREADS, 2)
         const TileCoord tc = tile_coord_t(in->g, in->ts, local, TZ, TY);
         const CUtensorMap* tmp = &in->tm[lit % 3];
         const CUtensorMap* tmc = &in->tm[(lit + 1) % 3];
+        if (BATCH && k != acquired) {
+          tmap_acquire(tmp);
+          tmap_acquire(tmc);
+          tmap_acquire(&in->tmm);
+          acquired = k;
+        }
         const uint32_t bbytes = TZ * TY * 8 * in->ncoef;
         for (int p = tc.x0 - 1; p <= tc.x1 && !*abort_flag; ++p) {
           const int sa = pa.s;

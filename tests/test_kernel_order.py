@@ -66,3 +66,16 @@ def test_cg_acquires_its_tensor_maps():
     kernel = _body(_source("sw_project.cu"), r"cg_ring\(const CgInst")
     assert 0 <= kernel.find("tmap_acquire(m)") < kernel.index("prefetch_tmap(m)")
     assert kernel.index("prefetch_tmap(m)") < kernel.index("ring_load<")
+
+
+@pytest.mark.parametrize("name,kernel", [
+    ("sw_step_tma.cu", r"step_f32_tma\(const"), ("sw_step_tma.cu", r"step_f64_tma\(const"),
+    ("sw_step_tb.cu", r"step_f32_fused2\(const")])
+def test_batched_steps_acquire_their_tensor_maps(name, kernel):
+    # a batch's maps lie in its table, whose room the next batch uses again
+    body = _body(_source(name), kernel)
+    at = body.index("if (BATCH && k != acquired)")
+    assert at < body.index("tma_load_4d(")
+    acquired = set(re.findall(r"tmap_acquire\(([^)]*)\)", body[at:]))
+    used = set(re.findall(r"tma_load_4d\([^,]*, ([^,]*),", body))
+    assert acquired == used
