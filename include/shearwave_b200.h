@@ -126,7 +126,8 @@ typedef struct sw_cg_stats {
   double max_div;  /* max |div_c f| of the masked input */
 } sw_cg_stats;
 
-/* Bytes of device workspace sw_project needs for an (nx, ny, nz) grid. */
+/* Bytes of device workspace sw_project needs for an (nx, ny, nz) grid (at any
+ * alignment, as all workspaces of the projections and the static solve). */
 size_t sw_project_workspace_bytes(int nx, int ny, int nz);
 
 /* Project (fx, fy, fz) onto discretely divergence-free fields in FP64.

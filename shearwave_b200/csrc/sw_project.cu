@@ -816,7 +816,10 @@ size_t cg_workspace_bytes(const Geom& g, const TileSpace& ts) {
   b += align_up((size_t)ts.count * sizeof(double2), 256);        // partials
   b += align_up(sizeof(CgState), 256);                           // state + grid barrier
   b += align_up(sizeof(CgInst), 256);                            // instance table
-  b += align_up(3 * sizeof(void*) + sizeof(InStride) + sizeof(double*), 256);
+  // input and output pointers, and the room of align_workspace
+  constexpr size_t ptrs = 3 * sizeof(void*) + sizeof(InStride) + sizeof(double*);
+  static_assert(ptrs + kWorkspaceAlign - 1 <= 256, "no room for align_workspace");
+  b += 256;
   return b;
 }
 
@@ -832,7 +835,7 @@ int cg_layout(const Geom& g, char* ws, size_t ws_bytes, CgInst* in, CgState** st
     return SW_EWORKSPACE;
   }
   size_t vec = align_up((size_t)g.ncell * sizeof(double), 256);
-  char* p = ws;
+  char* p = align_workspace(ws);
   in->x = (double*)p;
   p += vec;
   in->r = (double*)p;

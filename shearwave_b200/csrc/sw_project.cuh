@@ -63,6 +63,13 @@ struct CgInst {
 };
 
 size_t align_up(size_t v, size_t a);
+
+// Callers' workspaces may lie on any address.  The kernels' vectors and tensor
+// maps need 64-byte boundaries (TMA) and 16-byte ones (cp.async, pairs), so a
+// workspace is used from its first 128-byte boundary on; the last 256 bytes of
+// every workspace size leave the room for it.
+constexpr size_t kWorkspaceAlign = 128;
+inline char* align_workspace(char* ws) { return (char*)align_up((size_t)ws, kWorkspaceAlign); }
 TileSpace cg_tiles(const Geom& g);
 size_t cg_workspace_bytes(const Geom& g, const TileSpace& ts);
 

@@ -512,12 +512,15 @@ int spectral_one(const void* fx, const void* fy, const void* fz, InStride fs, co
                  double dX, double dY, double dZ, double* out, char* ws, size_t ws_bytes,
                  sw_cg_stats* stats, cudaStream_t s) {
   const size_t vec = align_up((size_t)g.ncell * sizeof(double), 256);
+  // (the last 256 bytes: the maximum, and the room of align_workspace)
   const size_t need = 3 * vec + spectral_extra_bytes(g) + 256;
+  static_assert(sizeof(double) + kWorkspaceAlign - 1 <= 256, "no room for align_workspace");
   if (ws == nullptr || ws_bytes < need) {
     set_error("spectral workspace of %zu bytes is smaller than the %zu bytes required", ws_bytes,
               need);
     return SW_EWORKSPACE;
   }
+  ws = align_workspace(ws);
   double* v0 = (double*)ws;
   double* v1 = (double*)(ws + vec);
   double* v2 = (double*)(ws + 2 * vec);
