@@ -580,9 +580,9 @@ class _Op:
 
     Those two Python kernels took 7 of the 20 us of a stencil operator's call
     and 30 of the 80 us of a time-loop op's (laplacian, divergence and gradient
-    of a 64^3 field: 100 -> 70 us).  Modes, fake tensors and function transforms still see the call; a
-    call that traces, or one with an argument that requires a gradient, takes
-    the whole path.
+    of a 64^3 field: 100 -> 70 us).  Modes, fake tensors and function transforms
+    still see the call; a call that traces, one with an argument that requires a
+    gradient, and one with keyword arguments take the whole path.
     """
 
     def __init__(self, op):
@@ -591,10 +591,10 @@ class _Op:
         self._written = [k for k, a in enumerate(self._overload._schema.arguments)
                          if a.alias_info is not None and a.alias_info.is_write]
 
-    def __call__(self, *args):
-        if torch.compiler.is_compiling() or (torch.is_grad_enabled()
-                                             and torch._C._any_requires_grad(*args)):
-            return self._op(*args)
+    def __call__(self, *args, **kwargs):
+        if kwargs or torch.compiler.is_compiling() or (torch.is_grad_enabled()
+                                                       and torch._C._any_requires_grad(*args)):
+            return self._op(*args, **kwargs)
         with torch._C._ExcludeDispatchKeyGuard(_GRADIENT_KEYS):
             out = self._overload(*args)
         for k in self._written:  # what the skipped kernels do for a written argument

@@ -53,3 +53,21 @@ def test_written_arguments_get_a_new_version(call):
         v0, s0 = dst._version, src._version
         call(dst, src, 1, [4, 4, 4], [0, 16, 4, 1], 1.0, None, [0, 0, 0])
         assert dst._version == v0 + 1 and src._version == s0
+
+
+def test_keyword_arguments():
+    with FakeTensorMode():
+        f = torch.empty((5, 6, 7), device="cuda")
+        assert ops.laplacian(f=f, h=[1.0, 1.0, 1.0]).shape == f.shape
+        assert ops.laplacian(f, h=[1.0, 1.0, 1.0]).shape == f.shape
+        out, st = ops.project(fx=f, fy=None, fz=None, h=[1.0] * 3, tol=1e-8, max_iters=4,
+                              method="cg")
+        assert out.shape == (3, 5 * 6 * 8) and st.shape == (4,)
+        dst = torch.empty((4, 4, 4), device="cuda")
+        v = dst._version
+        ops.convert_(dst=dst, src=torch.empty(128, device="cuda", dtype=torch.float64), ncomp=1,
+                     shape=[4, 4, 4], dst_strides=[0, 16, 4, 1], scale=1.0, rho=None,
+                     rho_strides=[0, 0, 0])
+        assert dst._version == v + 1
+    with pytest.raises(RuntimeError):
+        ops.laplacian(f, g=f)
