@@ -602,25 +602,38 @@ extern "C" int sw_convert(int ncomp, const double* src, int nx, int ny, int nz, 
     set_error("sw_convert: bad arguments");
     return SW_EINVAL;
   }
-  Geom g = make_geom(nx, ny, nz, pad_pitch(nz));
-  const dim3 grid((unsigned)((nz + TILE_Z - 1) / TILE_Z), (unsigned)((ny + TILE_Y - 1) / TILE_Y),
-                  (unsigned)((nx + kConvertPlanes - 1) / kConvertPlanes));
-  const dim3 block(TILE_Z, TILE_Y);
-  cudaStream_t s = (cudaStream_t)stream;
-#define SW_CONV(TO, TR)                                                                     \
-  convert_kernel<TO, TR><<<grid, block, 0, s>>>(ncomp, src, g, (TO*)dst, dst_cs, dst_sx, dst_sy, \
-                                              dst_sz, scale, (const TR*)rho, rho_sx, rho_sy,  \
-                                              rho_sz)
-  if (out_dtype == SW_F32 && rho_dtype == SW_F32) SW_CONV(float, float);
-  else if (out_dtype == SW_F32 && rho_dtype == SW_F64) SW_CONV(float, double);
-  else if (out_dtype == SW_F64 && rho_dtype == SW_F32) SW_CONV(double, float);
-  else if (out_dtype == SW_F64 && rho_dtype == SW_F64) SW_CONV(double, double);
-  else {
+  if ((out_dtype != SW_F32 && out_dtype != SW_F64) ||
+      (rho_dtype != SW_F32 && rho_dtype != SW_F64)) {
     set_error("sw_convert: unknown dtype");
     return SW_EINVAL;
   }
+  const Geom whole = make_geom(nx, ny, nz, pad_pitch(nz));
+  const dim3 block(TILE_Z, TILE_Y);
+  cudaStream_t s = (cudaStream_t)stream;
+  // one launch, unless the grid is longer along y or x than 65535 blocks are
+  constexpr int kMostY = 65535 * TILE_Y, kMostX = 65535 * kConvertPlanes;
+  for (long long y0 = 0; y0 < ny; y0 += kMostY)
+    for (long long x0 = 0; x0 < nx; x0 += kMostX) {
+      Geom g = whole;  // its strides, the slab's extents
+      g.ny = (int)std::min<long long>(kMostY, ny - y0);
+      g.nx = (int)std::min<long long>(kMostX, nx - x0);
+      const dim3 grid((unsigned)((nz + TILE_Z - 1) / TILE_Z),
+                      (unsigned)((g.ny + TILE_Y - 1) / TILE_Y),
+                      (unsigned)((g.nx + kConvertPlanes - 1) / kConvertPlanes));
+      const double* from = src + x0 * g.sxy + y0 * g.pz;
+      const long long to = x0 * dst_sx + y0 * dst_sy, at = x0 * rho_sx + y0 * rho_sy;
+#define SW_CONV(TO, TR)                                                                       \
+  convert_kernel<TO, TR><<<grid, block, 0, s>>>(ncomp, from, g, (TO*)dst + to, dst_cs, dst_sx,  \
+                                                dst_sy, dst_sz, scale,                        \
+                                                rho ? (const TR*)rho + at : nullptr, rho_sx,  \
+                                                rho_sy, rho_sz)
+      if (out_dtype == SW_F32 && rho_dtype == SW_F32) SW_CONV(float, float);
+      else if (out_dtype == SW_F32) SW_CONV(float, double);
+      else if (rho_dtype == SW_F32) SW_CONV(double, float);
+      else SW_CONV(double, double);
 #undef SW_CONV
-  count_launches(1);
-  SW_CHECK_LAUNCH("convert");
+      count_launches(1);
+      SW_CHECK_LAUNCH("convert");
+    }
   return SW_OK;
 }

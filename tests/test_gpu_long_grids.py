@@ -1,0 +1,35 @@
+"""Grids longer than a launch's 65535 blocks along y or x."""
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(262145, 1, 3), (1, 524281, 2), (262141, 2, 33)])
+def test_convert(cuda, shape):
+    import torch
+
+    from shearwave_b200 import ops
+
+    nx, ny, nz = shape
+    g = torch.Generator(device="cuda").manual_seed(4)
+    src = torch.randn((nx, ny, ops.pitch(nz)), device=cuda, dtype=torch.float64, generator=g)
+    dst = torch.full(shape, -7.0, device=cuda)
+    ops.convert_(dst, src.reshape(-1), 1, list(shape), [0, ny * nz, nz, 1], 0.5, None, [0, 0, 0])
+    assert torch.equal(dst, (src[..., :nz] * 0.5).float())
+
+
+def test_convert_in_strides_with_densities(cuda):
+    # two components into a (nx, ny, nz, 2) array, divided by a map's density
+    import torch
+
+    from shearwave_b200 import ops
+
+    nx, ny, nz = 262142, 3, 2
+    g = torch.Generator(device="cuda").manual_seed(9)
+    src = torch.randn((2, nx, ny, ops.pitch(nz)), device=cuda, dtype=torch.float64, generator=g)
+    rho = torch.rand((nx, ny, nz), device=cuda, dtype=torch.float64, generator=g) + 0.5
+    dst = torch.empty((nx, ny, nz, 2), device=cuda, dtype=torch.float64)
+    ops.convert_(dst, src.reshape(-1), 2, [nx, ny, nz], [1, ny * nz * 2, nz * 2, 2], 1.0, rho,
+                 [ny * nz, nz, 1])
+    assert torch.equal(dst, (src[..., :nz] * (1.0 / rho)).permute(1, 2, 3, 0).contiguous())
