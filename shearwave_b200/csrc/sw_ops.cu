@@ -239,7 +239,7 @@ template <typename T, bool PAIRS, bool AOS, bool ALL>
 __global__ void __launch_bounds__(kCellBlockZ * kCellBlockY)
     strain_kernel(const T* __restrict__ ux, const T* __restrict__ uy, const T* __restrict__ uz,
                   long long sx, long long sy, long long sz, Dense d, ConstDiv<T> h2x,
-                  ConstDiv<T> h2y, ConstDiv<T> h2z, ConstDiv<T> third, double vm_c,
+                  ConstDiv<T> h2y, ConstDiv<T> h2z, ConstDiv<T> third, double vm_c, int planes,
                   T* __restrict__ eps, T* __restrict__ vol, T* __restrict__ dev,
                   T* __restrict__ msh, double* __restrict__ vm) {
   using A = Ar<T>;
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(kCellBlockZ * kCellBlockY)
   const int z0 = blockIdx.x * kCellBlockZ, z = z0 + lane;
   const int y = blockIdx.y * kCellBlockY + threadIdx.y;
   if (y >= d.ny) return;  // whole warps
-  const int x0 = blockIdx.z * kStrainPlanes, x1 = min(x0 + kStrainPlanes, d.nx);
+  const int x0 = blockIdx.z * planes, x1 = min(x0 + planes, d.nx);
   const bool zin = z < d.nz, yin = y >= 1 && y <= d.ny - 2;
   const bool inner_zy = yin && z >= 1 && z <= d.nz - 2;
   const bool fast = h2x.fast && h2y.fast && h2z.fast;
@@ -399,10 +399,13 @@ ConstDiv<T> twice(double h) {
 }
 const double kVonMises = std::sqrt(2.0 / 3.0);
 int blocks_for(long long n) { return grid_blocks(n, 256, 148 * 32); }
+// planes per block: kStrainPlanes, more where they would take over 65535 blocks
+int strain_planes(int nx) { return std::max(kStrainPlanes, (nx - 1) / 65535 + 1); }
 dim3 strain_grid(int nx, int ny, int nz) {
+  const int planes = strain_planes(nx);
   return dim3((unsigned)((nz + kCellBlockZ - 1) / kCellBlockZ),
               (unsigned)((ny + kCellBlockY - 1) / kCellBlockY),
-              (unsigned)((nx + kStrainPlanes - 1) / kStrainPlanes));
+              (unsigned)((nx - 1) / planes + 1));
 }
 // whether a tensor's six values per cell can be read or written in pairs
 template <typename T>
@@ -431,7 +434,8 @@ void launch_strain(const void* ux, const void* uy, const void* uz, int64_t sx, i
   else fn = strain_kernel<T, true, false, false>;
   fn<<<strain_grid(d.nx, d.ny, d.nz), kCellBlock, 0, s>>>(
       (const T*)ux, (const T*)uy, (const T*)uz, sx, sy, sz, d, twice<T>(dX), twice<T>(dY),
-      twice<T>(dZ), const_div(T(3)), kVonMises, (T*)eps, (T*)vol, (T*)dev, (T*)msh, vm);
+      twice<T>(dZ), const_div(T(3)), kVonMises, strain_planes(d.nx), (T*)eps, (T*)vol, (T*)dev,
+      (T*)msh, vm);
 }
 
 template <typename T>

@@ -1,5 +1,6 @@
 """Grids longer than a launch's 65535 blocks along y or x."""
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +34,18 @@ def test_convert_in_strides_with_densities(cuda):
     ops.convert_(dst, src.reshape(-1), 2, [nx, ny, nz], [1, ny * nz * 2, nz * 2, 2], 1.0, rho,
                  [ny * nz, nz, 1])
     assert torch.equal(dst, (src[..., :nz] * (1.0 / rho)).permute(1, 2, 3, 0).contiguous())
+
+
+@pytest.mark.parametrize("shape", [(786421, 3, 3), (65536, 4, 3)])
+def test_strain(cuda, shape):
+    import shearwave_b200 as sw
+    from oracle import shearwave_oracle as O
+
+    rng = np.random.default_rng(6)
+    u = rng.standard_normal((*shape, 3), dtype=np.float32)
+    h = (0.5e-3, 0.37e-3, 0.71e-3)
+    ref = O.compute_strain_tensor(*np.moveaxis(u, -1, 0), *h)
+    eps, inv = sw.compute_strain_fields(u, *h)
+    assert np.array_equal(eps, ref)
+    for k, v in O.compute_strain_invariants(ref).items():
+        assert np.array_equal(inv[k], v), k
