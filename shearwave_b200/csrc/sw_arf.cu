@@ -35,10 +35,10 @@ constexpr int kEnvMaxThreads = 1024;
 
 template <typename T>
 __global__ void __launch_bounds__(kEnvMaxThreads, 2)
-    arf_env_partial(const T* __restrict__ p, long long ncell, int nt, int cn, int k,
+    arf_env_partial(const T* __restrict__ p, long long ncell, int nt, int chunk0, int cn, int k,
                     long long rows_per_block, double* __restrict__ partials) {
   extern __shared__ double env_red[];  // [k][cn]
-  const int cb = blockIdx.y * cn, w = min(cn, nt - cb);
+  const int cb = (chunk0 + blockIdx.y) * cn, w = min(cn, nt - cb);
   const int r = threadIdx.x / cn, c = threadIdx.x % cn;
   const long long r0 = (long long)blockIdx.x * rows_per_block;
   const long long r1 = r0 + rows_per_block < ncell ? r0 + rows_per_block : ncell;
@@ -392,8 +392,8 @@ extern "C" int sw_arf_envelope(int dtype, const void* p, int64_t ncell, int32_t 
   cudaStream_t s = (cudaStream_t)stream;
   // columns per block, and rows of them: the count that leaves the fewest
   // lanes of the last warp idle
-  const int chunks = (nt + kEnvMaxThreads - 1) / kEnvMaxThreads;
-  const int cn = (nt + chunks - 1) / chunks;
+  const int chunks = (nt - 1) / kEnvMaxThreads + 1;
+  const int cn = (nt - 1) / chunks + 1;
   int k = 1;
   double best = 0.0;
   for (int c = 1; c * cn <= kEnvMaxThreads && c <= 64; ++c) {
@@ -409,17 +409,21 @@ extern "C" int sw_arf_envelope(int dtype, const void* p, int64_t ncell, int32_t 
   const long long nblk = std::min(env_blocks(ncell), std::max(2LL, 4LL / chunks) * per_sm * kNumSMs);
   const long long rows = (ncell + nblk - 1) / nblk;
   const size_t smem = sizeof(double) * (size_t)k * cn;
-  const dim3 grid((unsigned)nblk, (unsigned)chunks);
   double* part = (double*)workspace;
-  if (dtype == SW_F32)
-    arf_env_partial<float><<<grid, threads, smem, s>>>((const float*)p, ncell, nt, cn, k, rows,
-                                                       part);
-  else
-    arf_env_partial<double><<<grid, threads, smem, s>>>((const double*)p, ncell, nt, cn, k, rows,
-                                                        part);
+  // one launch, unless a record has more than 65535 chunks
+  for (int c0 = 0; c0 < chunks; c0 += 65535) {
+    const dim3 grid((unsigned)nblk, (unsigned)std::min(chunks - c0, 65535));
+    if (dtype == SW_F32)
+      arf_env_partial<float><<<grid, threads, smem, s>>>((const float*)p, ncell, nt, c0, cn, k,
+                                                         rows, part);
+    else
+      arf_env_partial<double><<<grid, threads, smem, s>>>((const double*)p, ncell, nt, c0, cn, k,
+                                                          rows, part);
+    count_launches(1);
+  }
   arf_env_final<<<(nt + kEnvFinal - 1) / kEnvFinal, dim3(kEnvFinal, kEnvFinal), 0, s>>>(
       part, (int)nblk, nt, ncell, env);
-  count_launches(2);
+  count_launches(1);
   SW_CHECK_LAUNCH("radiation-force envelope");
   return SW_OK;
 }

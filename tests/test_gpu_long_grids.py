@@ -1,4 +1,5 @@
-"""Grids longer than a launch's 65535 blocks along y or x."""
+"""Grids longer than a launch's 65535 blocks along y or x, and records longer than that
+many chunks of samples."""
 
 import numpy as np
 import pytest
@@ -49,3 +50,18 @@ def test_strain(cuda, shape):
     assert np.array_equal(eps, ref)
     for k, v in O.compute_strain_invariants(ref).items():
         assert np.array_equal(inv[k], v), k
+
+
+@pytest.mark.parametrize("ncell", [1, 3])
+def test_envelope(cuda, ncell):
+    import torch
+
+    from shearwave_b200 import ops
+
+    nt = 65535 * 1024 + 5
+    g = torch.Generator(device="cuda").manual_seed(8)
+    p = torch.randint(-8, 9, (ncell, nt), device=cuda, generator=g, dtype=torch.int8).float()
+    env = ops.arf_envelope(p, ncell, nt)
+    # whole numbers: every sum is exact, the division rounded once (by numpy: torch
+    # multiplies by the reciprocal)
+    assert np.array_equal(env.cpu().numpy(), (p.double() ** 2).sum(0).cpu().numpy() / ncell)
