@@ -829,8 +829,9 @@ def shear_fdtd(
     "spectral" explicitly), ``kahan`` (False: compensated displacement sum), ``step_kernel`` ("tma" default, or "direct"), ``xchunk`` (planes
     per tile along x, 0 = automatic), ``steps_per_pass`` (mixed form: 2
     fuses two time steps per pass over HBM, except with ``kahan``; 1 one
-    step per launch; 0 (default) two), ``cuda_graph`` (True: long step runs are resident launches of the two-step
-    kernel or replay one instantiated CUDA graph of 32 steps; False: one launch
+    step per launch; 0 (default) two), ``cuda_graph`` (True: long step runs are
+    resident launches of the two-step kernel, which hold the GPU for about 2 ms
+    each, or replay one instantiated CUDA graph of 32 steps; False: one launch
     at a time), ``force_terms`` (extra separable terms:
     list of ``((bx, by, bz), env)``), ``force_stream_bytes`` (4-D forces: the
     non-zero slices are projected up front and streamed from the device

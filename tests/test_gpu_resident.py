@@ -86,3 +86,27 @@ def test_two_streams(cuda):
     torch.cuda.synchronize()
     for o, r in zip(outs, ref):
         assert all(torch.equal(x, y) for x, y in zip(o, r))
+
+
+@pytest.mark.parametrize("shape,n_steps", [((64, 64, 64), 762), ((256, 256, 384), 48)])
+def test_a_launch_holds_the_gpu_for_about_two_milliseconds(cuda, shape, n_steps):
+    """Work on other streams waits for a resident launch, so its length is bounded."""
+    import torch
+
+    from shearwave_b200 import _native, ops
+    from shearwave_b200 import solver as S
+
+    b = torch.ones(shape, device=cuda)
+    sv = S._Solve(None, None, b, 1000.0, 2000.0, 1e-3, 1e-3, 1e-3, 1e-5, n_steps,
+                  dict(env_t=np.zeros(n_steps, np.float32), poisson_tol=1e-10))
+    S._project_inputs([sv])
+    sv.build_terms()
+    sv.run_loop(None)  # warm
+    ends = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    torch.cuda.synchronize()
+    n = _native.launch_count()
+    ends[0].record()
+    ops.fdtd_steps_(*sv.run.bundle(), 0, n_steps)
+    ends[1].record()
+    torch.cuda.synchronize()
+    assert ends[0].elapsed_time(ends[1]) / (_native.launch_count() - n) < 3.0
