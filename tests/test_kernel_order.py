@@ -79,3 +79,14 @@ def test_batched_steps_acquire_their_tensor_maps(name, kernel):
     acquired = set(re.findall(r"tmap_acquire\(([^)]*)\)", body[at:]))
     used = set(re.findall(r"tma_load_4d\([^,]*, ([^,]*),", body))
     assert acquired == used
+
+
+def test_cg_frees_a_unit_after_its_points():
+    # the points' room has no barrier of its own: it is used again on the word
+    # of the unit's stage
+    tile = _body(_source("sw_project.cu"), r"bool ring_tile\([^{]*")
+    walk = _body(tile, r"for \(int j = 0; j < n; j \+= 2[^{]*")
+    assert walk.count("release(") == 1
+    reads = [m.start() for m in re.finditer(r"finish\(c[01], ap[01], B", walk)]
+    assert len(reads) == 2 and "q.points()" in walk[:reads[0]]
+    assert walk.index("release(s0)") > max(reads)
