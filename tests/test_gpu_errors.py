@@ -157,3 +157,44 @@ def test_single_solve_timeout(cuda, precision, n_steps):
                             p["dZ"], p["dT"], p["n_steps"], dict(p["opts"], precision=precision))
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
+
+
+def test_lone_mixed_solve_resident_and_replayed(cuda):
+    """A lone mixed solve of long chunks steps in resident launches, without a tile
+    queue in replays of one graph: the same results, and the same end when a wait
+    runs out.  (The smaller grids above have chunks of one plane, which no resident
+    launch takes.)"""
+    import torch
+
+    import shearwave_b200._native as native
+    from shearwave_b200 import solver as S
+    from shearwave_b200 import workloads as W
+
+    def run(resident, stall=False):
+        sv = _solves([W.problem_inclusions((64, 48, 70), 80, seed=310, tol=1e-9)], "mixed")[0]
+        S._project_inputs([sv])
+        sv.build_terms()
+        sv.run.stall_test = int(stall)
+        if not resident:
+            sv.run.queue = None
+        calls, kernels = native.host_enqueue_count(), native.launch_count()
+        sv.run_loop(None)
+        calls, kernels = native.host_enqueue_count() - calls, native.launch_count() - kernels
+        torch.cuda.synchronize()
+        return sv, calls, kernels
+
+    ref, calls, kernels = run(True)
+    assert kernels < 10  # many pairs each
+    got, calls, kernels = run(False)
+    assert kernels >= 40 and calls < kernels  # a launch per pair, replayed
+    assert torch.equal(got.run.state, ref.run.state)
+    for resident in (True, False):
+        with _wait_budget(SHORT_BUDGET):
+            sv, _, _ = run(resident, stall=True)
+            rc, flags = _status(sv)
+        assert rc == native.SW_ETIMEOUT and flags & native.FLAG_TIMEOUT
+        # the progress words and the queue are zero for the next launch
+        assert int(torch.count_nonzero(sv.run.state[:, 6:])) == 0
+        assert sv.run.queue is None or sv.run.queue.tolist() == [0, 0]
+    again, _, _ = run(True)
+    assert torch.equal(again.run.state, ref.run.state)
