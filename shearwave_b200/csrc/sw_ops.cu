@@ -7,7 +7,9 @@
 // These kernels reproduce numpy's elementwise rounding: every operation is a
 // separately rounded IEEE operation in the array dtype (no FMA contraction,
 // true division by the same divisor numpy uses), so their outputs equal the
-// reference's bit for bit in float32 and float64.
+// reference's bit for bit in float32 and float64.  One exception: where the
+// second invariant is NaN (a strain that overflowed), max_shear is 0; numpy's
+// maximum keeps the NaN, as the other invariants do here too.
 #include <math.h>
 
 #include <algorithm>

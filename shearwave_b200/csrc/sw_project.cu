@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(TILE_THREADS) cg_prep(const CgInst* __restrict
 // from shared memory.  The update phase walks x the other way, starting with
 // the planes the apply phase left in L2.  Two blocks per SM.  Measured against
 // a walk with every stencil point from global memory: an iteration at 192^3
-// takes 86 instead of 160 us (DRAM bytes alone 69; 6 TB/s while the tiles
+// takes 84 instead of 160 us (DRAM bytes alone 69; 6 TB/s while the tiles
 // walk, the rest is the phases' ends), the 442 of a static solve at 121 x 121
-// x 141, whose vectors fit L2, 13.6 instead of 31.6 ms.
+// x 141, whose vectors fit L2, 13.0 instead of 31.6 ms.
 // The walk goes by units of two planes (one barrier, and two independent
 // stencils for a thread to overlap).  Stages: the unit in work and the one
 // ahead held, two in flight.  A stage holds the boxes of p and r in the apply

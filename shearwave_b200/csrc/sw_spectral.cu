@@ -118,13 +118,16 @@ __global__ void axis_basis_kernel(int n, double h, AxisBasis ax) {
 // data once and pads its modes to a multiple of 32 only.  Measured: 64 x 64
 // tiles of the full n x n matrices with 8-byte loads and no pipeline, then
 // multiply-adds on the chains, then this: the six transforms of a 160 x 131 x
-// 173 grid 1154, 339, 246 us (whole projection 1406, 523, 426 us), the 48 of
+// 173 grid 1154, 339, 246 us (whole projection 1406, 523, 390 us), the 48 of
 // eight 256 x 256 x 384 forces 75.4, 21.0, 15.0 ms (axes x and y at 28
 // TFLOP/s of the multiply-adds a chain needs, axis z at 20).
 constexpr int SG_K = 16, SG_STAGES = 3;
 constexpr int SG_PAD = 8;  // rows 64 bytes apart modulo 128: the four depths of a fragment
-// resident blocks per SM: 16 to 18 warps (a multiply-add's latency is covered
-// by a thread's 32 accumulators; more warps cover the copies and barriers)
+// Resident blocks per SM that the registers are held to: 16 to 18 warps (a
+// multiply-add's latency is covered by a thread's 32 accumulators; more warps
+// cover the copies and barriers).  Shared memory leaves spec_rows 5, 4, 3, 2
+// blocks (10 to 18 warps) for WM 1 to 4, and spec_lines, whose rings hold both
+// chains, 4, 2, 2, 1 (8 to 12 warps).
 #define SG_BLOCKS(WM) ((WM) == 1 ? 8 : (WM) == 2 ? 4 : (WM) == 3 ? 3 : 2)
 
 __device__ __forceinline__ void cp_async8(void* dst, const void* src, bool ok) {

@@ -24,7 +24,7 @@
 // 0 of planes q-1 and q, level 1 of planes q-1 and q, the coefficients of
 // q-1) and takes the z neighbours from the lanes either side, so shared
 // memory serves only the rows either side, the column's next level-0 plane,
-// its level 1 of plane q-2 and the coefficients: 36 eight-byte loads per pair
+// its level 1 of plane q-2 and the coefficients: 38 eight-byte loads per pair
 // and plane instead of the 76 of reading every stencil point.  Plane q-2 comes
 // from the ring, where the thread itself wrote it, because with it in
 // registers too the loop cannot be unrolled by two without spilling, and
