@@ -271,9 +271,9 @@ typedef struct sw_fdtd_desc {
   /* Device int the step loop may use as its step counter: with it, long runs
    * of sw_fdtd_steps replay one instantiated CUDA graph of 32 steps instead
    * of launching every step (NULL: direct launches only).  With `queue` as
-   * well, pairs of steps of the F32 form run in resident launches, each of 2
-   * to 250 pairs and about 2 ms, in which it holds every SM (a grid whose pair
-   * takes over 1 ms gets a launch a pair); their progress words lie in the x = 0 shell plane of
+   * well, pairs of steps of the F32 form run in resident launches, each of 1
+   * to 250 pairs and about 2 ms (or the one pair), in which it holds every SM;
+   * their progress words lie in the x = 0 shell plane of
    * component 6 of state[0], and are zero again when a call's work is done. */
   int32_t* clock;
   /* Two device int32s, zero at the first call (the kernels leave them zero):

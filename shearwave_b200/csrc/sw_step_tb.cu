@@ -907,10 +907,10 @@ static int tb_resident_slots(int lz) {
 // state buffer 0, which is zero in every state and is cleared again, so the
 // solve's own memory carries them: any number of solves, streams and threads.
 // A launch holds every SM until it ends, and work on other streams waits for it,
-// so it is bounded to about 2 ms: 2 to 250 pairs by the time of one (a pair
-// measured 12 us at 64^3, 106 at 192^3, 0.42 ms at 256 x 256 x 384).
-// *done: steps enqueued, 0 when the solve's tiles do not allow it or one pair
-// takes more than half of that.
+// so it is bounded to about 2 ms, or one pair where that takes longer: 1 to 250
+// pairs by the time of one (a pair measured 12 us at 64^3, 106 at 192^3, 0.42 ms
+// at 256 x 256 x 384).  *done: steps enqueued, 0 when the solve's tiles do not
+// allow it.
 constexpr double kResidentUs = 2000.0;
 inline double pair_us(long long cells) { return 8.0 + 1.55e-5 * (double)cells; }
 int run_fused2_resident(const TmaF32TB& t, int* queue, int it0, int nsteps, cudaStream_t s,
@@ -921,8 +921,8 @@ int run_fused2_resident(const TmaF32TB& t, int* queue, int it0, int nsteps, cuda
   if (queue == nullptr || pairs < 2 || ntiles == 0 || (t.ts.xc < 2 && t.ts.nxc > 1)) return SW_OK;
   const int stride = (int)std::min<long long>(8, t.g.sxy / ntiles);
   if (stride < 1) return SW_OK;
-  const int most = (int)(kResidentUs / pair_us((long long)t.g.nx * t.g.ny * t.g.nz));
-  if (most < 2) return SW_OK;
+  const int most =
+      std::max(1, (int)(kResidentUs / pair_us((long long)t.g.nx * t.g.ny * t.g.nz)));
   const int slots = tb_resident_slots(t.lz);
   if (slots == 0) return SW_OK;
   const int grid = std::min(ntiles, slots);

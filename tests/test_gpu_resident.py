@@ -110,3 +110,29 @@ def test_a_launch_holds_the_gpu_for_about_two_milliseconds(cuda, shape, n_steps)
     ends[1].record()
     torch.cuda.synchronize()
     assert ends[0].elapsed_time(ends[1]) / (_native.launch_count() - n) < 3.0
+
+
+def test_a_pair_longer_than_the_bound(cuda):
+    """Grids whose pairs take over 2 ms keep resident launches, of one pair each."""
+    import torch
+
+    from shearwave_b200 import _native
+    from shearwave_b200 import solver as S
+
+    n_steps, states = 6, []
+    g = torch.Generator(device="cuda").manual_seed(3)
+    b = torch.randn((512, 512, 500), device=cuda, generator=g)
+    for resident in (True, False):
+        sv = S._Solve(None, None, b, 1000.0, 2000.0, 1e-3, 1e-3, 1e-3, 1e-5, n_steps,
+                      dict(env_t=np.ones(n_steps, np.float32), poisson_tol=1e-10))
+        S._project_inputs([sv])
+        sv.build_terms()
+        if not resident:
+            sv.run.queue = None
+        n = _native.launch_count()
+        sv.run_loop(None)
+        torch.cuda.synchronize()
+        assert n_steps // 2 <= _native.launch_count() - n < 10
+        assert int(torch.count_nonzero(sv.run.state[:, 6:])) == 0
+        states.append(sv.run.state)
+    assert torch.equal(*states)
